@@ -19,6 +19,7 @@
 // fixed order that the CPU restatement mirrors, so keys are bit-exact.
 #include "fvgs_device.cuh"
 #include "fvgs_launch.h"
+#include "pose_derivs.cuh"
 
 namespace fvgs {
 
@@ -35,6 +36,7 @@ __device__ __forceinline__ void add_rect(int* d, int gw, int x0, int y0, int x1,
 // previous binning (incremental mode), R and tw the camera pose; grid: the
 // count and entering difference grids (a.tile_diff, or the CTA's copy in
 // shared memory).
+template <bool DERIV>
 __device__ __forceinline__ void project_one(const ProjectArgs& a, int i, float4 p, uint32_t prev_count,
                                             const float (&R)[3][3], const float (&tw)[3], int* grid) {
     const fvgs_intrinsics K = a.K;
@@ -169,14 +171,13 @@ __device__ __forceinline__ void project_one(const ProjectArgs& a, int i, float4 
     if (count && (visible || (a.quirks & FVGS_Q_CULLED_SLOTS))) {
         const float4 co = a.attr_c ? unpack_c(a.attr_c[i]) : a.col[i];
         const bool swap = (a.quirks & FVGS_Q_INVSIGMA_SWAP) != 0;
-        a.rec0[i] = make_float4(u, v, z, co.w);
-        a.rec1[i] = make_float4(ixx, swap ? iyy : ixy, swap ? ixy : iyy, phx);
+        const float4 r0 = make_float4(u, v, z, co.w);
+        const float4 r1 = make_float4(ixx, swap ? iyy : ixy, swap ? ixy : iyy, phx);
+        a.rec0[i] = r0;
+        a.rec1[i] = r1;
         a.rec2[i] = make_float4(phy, co.x, co.y, co.z);
         a.bins[i].p = make_float4(u, v, z, phx);
-        if (a.geo0) {
-            a.geo0[i] = geo0;
-            a.geo1[i] = geo1;
-        }
+        if constexpr (DERIV) pose_derivs(K.fx, K.fy, swap, r0, r1, geo0, geo1, a.deriv + 8 * (size_t)i);
     }
     // bins[i].r.z == counts[i] after every binning; a Gaussian without
     // instances before and now needs no write (most of a large map).
@@ -309,6 +310,8 @@ __device__ __forceinline__ bool cand_reusable(const CandState& c, const DevPose&
     return fabsf(d) * rsqrtf(n0 * n1) >= cosf(0.5f * kCandMaxAngle);
 }
 
+// DERIV: the pose derivatives too (a.deriv, the analytic pose Jacobian).
+template <bool DERIV>
 __global__ void __launch_bounds__(kProjThreads, 4) project_count_kernel(ProjectArgs a) {
     pdl_begin();
     __shared__ uint32_t q_i[kProjChunk], q_prev[kProjChunk];
@@ -406,7 +409,7 @@ __global__ void __launch_bounds__(kProjThreads, 4) project_count_kernel(ProjectA
         const int nq = q_n;
         for (int k = threadIdx.x; k < nq; k += kProjThreads) {
             const uint32_t i = q_i[k];
-            project_one(a, (int)i, a.pos[i], q_prev[k], R, tw, grid);
+            project_one<DERIV>(a, (int)i, a.pos[i], q_prev[k], R, tw, grid);
         }
         __syncthreads();  // the queue is consumed before the next chunk's
     }
@@ -930,7 +933,7 @@ cudaError_t launch_copy_lists(const uint2* ranges, int T, const uint32_t* src, u
 cudaError_t launch_project_count(const ProjectArgs& a, int max_ctas, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
     const int need = (a.n + kProjChunk - 1) / kProjChunk;
-    return launch_chained(project_count_kernel, dim3(max_ctas > 0 && max_ctas < need ? max_ctas : need), dim3(256), 0,
+    return launch_chained(a.deriv ? project_count_kernel<true> : project_count_kernel<false>, dim3(max_ctas > 0 && max_ctas < need ? max_ctas : need), dim3(256), 0,
                           s, a);
 }
 

@@ -17,7 +17,6 @@
 #include <new>
 #include <vector>
 
-#include <cudaTypedefs.h>
 
 #include "../../include/fvgs.h"
 #include "fvgs_device.cuh"
@@ -144,9 +143,9 @@ struct fvgs_session {
 
     float4 *pos = nullptr, *scale = nullptr, *rot = nullptr, *col = nullptr;
     float4 *rec0 = nullptr, *rec1 = nullptr, *rec2 = nullptr;
-    // geometry records of the analytic pose Jacobian (sessions whose quirks
-    // clear FVGS_Q_POSE_JAC_APPROX): camera-frame covariance and mean
-    float4 *geo0 = nullptr, *geo1 = nullptr;
+    // pose derivatives of the analytic pose Jacobian (sessions whose quirks
+    // clear FVGS_Q_POSE_JAC_APPROX), 8 vectors per Gaussian
+    float4* deriv = nullptr;
     BinRec* bins = nullptr;  // binning records; bins[i].r.z == counts[i] after every binning
     uint32_t *counts = nullptr, *offsets = nullptr, *partials = nullptr;
     // the projection's candidate list (Gaussians that may be in view near the
@@ -248,8 +247,6 @@ struct fvgs_session {
     // colour/opacity that the projection reads; the float4 planes stay the
     // master copy (mapping updates both)
     // tensor maps of the record planes (TMA-staged Jacobian variant)
-    RecMaps rec_maps{};
-    bool rec_maps_ok = false;
 
     int precision = FVGS_PRECISION_FP32;
     bool autotune = true;  // tune the Jacobian kernel's launch variant on a frame shape's first frame
@@ -367,37 +364,6 @@ void dev_free(fvgs_session* s, T*& p, size_t count) {
         int r_ = (expr);        \
         if (r_ != FVGS_OK) return r_; \
     } while (0)
-
-// Tensor maps of the three record planes for the TMA-staged Jacobian kernel:
-// 2-D, 4 floats x capacity rows of 16 bytes, one-row boxes (gather4 loads).
-// The encoder comes from the driver through the runtime; without it the
-// variant is simply not offered.
-bool encode_record_maps(fvgs_session* s) {
-    static PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
-    static bool looked = false;
-    if (!looked) {
-        looked = true;
-        cudaDriverEntryPointQueryResult q{};
-        void* fn = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            enc = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-        cudaGetLastError();
-    }
-    if (!enc) return false;
-    float4* planes[3] = {s->rec0, s->rec1, s->rec2};
-    const cuuint64_t dims[2] = {4, (cuuint64_t)s->cap_g};
-    const cuuint64_t strides[1] = {sizeof(float4)};
-    const cuuint32_t box[2] = {4, 1};
-    const cuuint32_t elem[2] = {1, 1};
-    for (int p = 0; p < 3; ++p)
-        if (enc(&s->rec_maps.rec[p], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, planes[p], dims, strides, box, elem,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return false;
-    return true;
-}
 
 // Bring the reduced-precision planes up to date with the master planes after
 // a host-side map change (upload, removal, seeding).
@@ -650,8 +616,10 @@ float view_cone(const fvgs_intrinsics* K, int W, int H) {
     return (float)std::atan(std::sqrt(ex * ex + ey * ey));
 }
 
-// Enqueue binning for the pose already in s->pose.
-int enqueue_bin(fvgs_session* s, const fvgs_intrinsics* K, int W, int H, int tw, int th) {
+// Enqueue binning for the pose already in s->pose.  track: a tracking launch
+// follows, so the projection also writes the pose derivatives (sessions with
+// the analytic Jacobian).
+int enqueue_bin(fvgs_session* s, const fvgs_intrinsics* K, int W, int H, int tw, int th, bool track = false) {
     const fvgs_params& P = s->params;
     if (!track_tile_supported(tw, th)) return FVGS_E_INVALID;
     const int ntx = (W + tw - 1) / tw;
@@ -697,8 +665,7 @@ int enqueue_bin(fvgs_session* s, const fvgs_intrinsics* K, int W, int H, int tw,
     pa.rec2 = s->rec2;
     pa.bins = s->bins;
     pa.counts = s->counts;
-    pa.geo0 = s->geo0;
-    pa.geo1 = s->geo1;
+    pa.deriv = track ? s->deriv : nullptr;
     pa.cst = s->cst;
     if (!(s->debug & FVGS_DEBUG_NO_CANDIDATES)) pa.cand = s->cand;
     pa.cone = view_cone(K, W, H);
@@ -855,21 +822,18 @@ TrackArgs make_track_args(fvgs_session* s, const fvgs_intrinsics* K, const Frame
     }
     ta.render_only = render_only ? 1 : 0;
     ta.quirks = P.quirks;
-    ta.geo0 = s->geo0;
-    ta.geo1 = s->geo1;
+    ta.deriv = s->deriv;
     // precision form: the analytic Jacobian's accumulations compensated (16 x 16 tiles)
     ta.compensated = (s->precision == FVGS_PRECISION_REDUCED && !render_only &&
                       !(P.quirks & FVGS_Q_POSE_JAC_APPROX) && ta.tile_w == 16 && ta.tile_h == 16)
                          ? 1
                          : 0;
     ta.variant = (f.tuned_w == f.W && f.tuned_h == f.H) ? f.track_variant : 0;
-    if (ta.variant == 2 && !s->rec_maps_ok) ta.variant = 0;
     ta.split = 1;
     if (track_variant_split(ta.variant) > 1) {
         if (split_ok(ta)) ta.split = track_variant_split(ta.variant);
-        else ta.variant = 3;  // the same staging batch, one CTA per tile
+        else ta.variant = 0;
     }
-    ta.st_flags = &s->st->flags;
     return ta;
 }
 
@@ -878,7 +842,7 @@ int enqueue_track(fvgs_session* s, const fvgs_intrinsics* K, const FrameLevel& f
     const TrackArgs ta = make_track_args(s, K, f, render_only, images);
     if (!render_only) s->last_split = ta.split;
     KScope k(s, render_only ? FVGS_K_RENDER : FVGS_K_TRACK, 1);
-    FV_CK(launch_track(ta, s->rec_maps_ok ? &s->rec_maps : nullptr, s->stream));
+    FV_CK(launch_track(ta, s->stream));
     return FVGS_OK;
 }
 
@@ -1121,8 +1085,7 @@ int fvgs_session_create(const fvgs_params* params, int device, uint32_t capacity
     FV_A(s->rec1, N);
     FV_A(s->rec2, N);
     if (!(P.quirks & FVGS_Q_POSE_JAC_APPROX)) {
-        FV_A(s->geo0, N);
-        FV_A(s->geo1, N);
+        FV_A(s->deriv, 8 * N);
     }
     FV_A(s->offsets, N);
     FV_A(s->cst_all, kBinCtx);
@@ -1155,9 +1118,9 @@ int fvgs_session_create(const fvgs_params* params, int device, uint32_t capacity
     FV_A(s->changed, (size_t)s->enter_cap);
     FV_A(s->seg.large_list, (size_t)s->cap_tiles);
     FV_A(s->seg.large_ctrl, 4);  // [0..1] large-bucket list control, [2] scatter chunk counter
-    // partial rows: a tile of the smallest tracking tile each, or four per
-    // 16 x 16 tile split over 8 x 8 CTAs
-    FV_A(s->tile_out, (size_t)std::max(s->cap_tiles, 4 * s->cap_tiles16) * FVGS_POSEDATA_FLOATS);
+    // partial rows: four per tile (16 x 16 tiles run as 8 x 8 quarters), for
+    // as many tiles as a frame may have
+    FV_A(s->tile_out, 4 * (size_t)s->cap_tiles * FVGS_POSEDATA_FLOATS);
     FV_A(s->pose, 1);
     FV_A(s->d_pose_in, 1);
     FV_A(s->jj, 48);
@@ -1193,7 +1156,6 @@ int fvgs_session_create(const fvgs_params* params, int device, uint32_t capacity
         return fail(FVGS_E_NOMEM);
     if (cudaEventCreateWithFlags(&s->frame_done, cudaEventDisableTiming) != cudaSuccess) return fail(FVGS_E_CUDA);
     if (sort_init(&s->sort, device) != cudaSuccess) return fail(FVGS_E_CUDA);
-    s->rec_maps_ok = encode_record_maps(s);
     const uint64_t cap0 = std::max<uint64_t>(1u << 20, 8ull * N);
     if ((rc = alloc_instances(s, std::min<uint64_t>(cap0, 0xffffffffull))) != FVGS_OK) return fail(rc);
     if (cudaMemsetAsync(s->st, 0, sizeof(DevStatus), s->stream) != cudaSuccess) return fail(FVGS_E_CUDA);
@@ -1576,7 +1538,7 @@ int fvgs_track_jacobian(fvgs_session* s, const fvgs_pose* pose, const fvgs_intri
     for (int attempt = 0; attempt < 4; ++attempt) {
         FV_TRY(reset_status(s));
         FV_TRY(set_pose(s, pose));
-        FV_TRY(enqueue_bin(s, K, f.W, f.H, f.tile_w, f.tile_h));
+        FV_TRY(enqueue_bin(s, K, f.W, f.H, f.tile_w, f.tile_h, true));
         FV_TRY(enqueue_track(s, K, f, false, images));
         {
             KScope k(s, FVGS_K_REDUCE, 1);
@@ -1642,10 +1604,8 @@ namespace {
 // of this shape.  Every variant computes the same values in the same order,
 // so the choice changes only the time.
 // Whether launch variant v is a distinct choice for the level's frames: the
-// TMA-staged one needs the record tensor maps; the split ones need 16 x 16
-// tiles without compensated sums.
+// split ones need 16 x 16 tiles without compensated sums.
 bool variant_applies(const fvgs_session* s, const FrameLevel& f, int v) {
-    if (v == 2) return s->rec_maps_ok;
     if (track_variant_split(v) > 1) {
         TrackArgs a{};
         a.tile_w = f.tile_w ? f.tile_w : 16;
@@ -1664,7 +1624,7 @@ int autotune_track(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics
         if (attempt == 4) return FVGS_E_CAPACITY;
         FV_TRY(reset_status(s));
         FV_TRY(set_pose(s, pose));
-        FV_TRY(enqueue_bin(s, K, f.W, f.H, f.tile_w, f.tile_h));
+        FV_TRY(enqueue_bin(s, K, f.W, f.H, f.tile_w, f.tile_h, true));
         FV_CK(cudaMemcpyAsync(s->h_st, s->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, s->stream));
         FV_CK(cudaStreamSynchronize(s->stream));
         collect_timing(s);
@@ -1748,7 +1708,7 @@ int fvgs_session_set_autotune(fvgs_session* s, int enabled) {
 int fvgs_session_set_track_variant(fvgs_session* s, int level, int variant) {
     if (!s || level < 0 || level >= kMaxLevels || variant < 0 || variant >= kTrackVariants) return FVGS_E_INVALID;
     FrameLevel& f = s->lv[level];
-    if (!f.rgb || (variant == 2 && !s->rec_maps_ok)) return FVGS_E_STATE;
+    if (!f.rgb) return FVGS_E_STATE;
     f.track_variant = variant;
     f.tuned_w = f.W;
     f.tuned_h = f.H;
@@ -1770,7 +1730,7 @@ int enqueue_frame(fvgs_session* s, const fvgs_session::FrameRequest& r) {
     for (int l = kMaxLevels - 1; l >= 0; --l) {
         const FrameLevel& f = s->lv[l];
         for (int it = 0; it < r.iters[l]; ++it) {
-            FV_TRY(enqueue_bin(s, &r.K[l], f.W, f.H, f.tile_w, f.tile_h));
+            FV_TRY(enqueue_bin(s, &r.K[l], f.W, f.H, f.tile_w, f.tile_h, true));
             FV_TRY(enqueue_track(s, &r.K[l], f, false, false));
             KScope k(s, FVGS_K_GN, 1);
             FV_CK(launch_track_reduce_gn(s->tile_out, s->last_T, s->last_split, s->pose, s->jj, s->params.eig_eps,
@@ -2185,7 +2145,7 @@ struct fvgs_batch {
         BinSnap entry, exit;  // the session's binning contexts before and after the frame
         int W[kMaxLevels] = {}, H[kMaxLevels] = {};
         fvgs_intrinsics K[kMaxLevels] = {};
-        int tw = 0, th = 0, last_W = 0, last_H = 0, last_T = 0;
+        int tw = 0, th = 0, last_W = 0, last_H = 0, last_T = 0, last_split = 1;
         uint64_t launches[FVGS_K_COUNT] = {};
     };
     struct Graph {
@@ -2245,14 +2205,14 @@ int batch_ensure_tables(fvgs_batch* b, int iters) {
     return FVGS_OK;
 }
 
-// Push a level's tile shape and staging batch to every session, so each one's
-// plain frames blend exactly as the batch does.
+// Push a level's tile shape to every session, so each one's plain frames
+// blend exactly as the batch does.
 void batch_apply_level(fvgs_batch* b, int l) {
     for (fvgs_session* s : b->s) {
         FrameLevel& f = s->lv[l];
         f.tile_w = b->tw[l];
         f.tile_h = b->th[l];
-        f.track_variant = b->variant[l];
+        f.track_variant = 0;
         f.tuned_w = f.W;
         f.tuned_h = f.H;
         ++s->gen;
@@ -2283,17 +2243,19 @@ int batch_bin_level(fvgs_batch* b, const Request* reqs, int l, int it, uint32_t*
     for (size_t i = 0; i < n; ++i) {
         fvgs_session* s = b->s[i];
         const FrameLevel& f = s->lv[l];
-        FV_TRY(enqueue_bin(s, &reqs[i].K[l], f.W, f.H, b->tw[l], b->th[l]));
+        FV_TRY(enqueue_bin(s, &reqs[i].K[l], f.W, f.H, b->tw[l], b->th[l], true));
         TrackJob& j = b->h_jobs[(size_t)it * n + i];
         j.a = make_track_args(s, &reqs[i].K[l], f, false, false);
-        j.a.variant = b->variant[l];
-        j.a.split = 1;  // the persistent launch runs one work item per tile
+        // the persistent launch runs one work item per tile, or per 8 x 8
+        // quarter of a 16 x 16 tile
+        const int split = track_batch_split(b->tw[l], b->th[l]);
+        j.a.split = s->last_split = split;
         b->h_begin[(size_t)it * (n + 1) + i] = t;
-        t += (uint32_t)s->last_T;
+        t += (uint32_t)(s->last_T * split);
         ReduceJob& r = b->h_rjobs[(size_t)it * n + i];
         r.tile_out = s->tile_out;
         r.num_tiles = s->last_T;
-        r.split = 1;
+        r.split = split;
         r.pose = s->pose;
         r.out = s->jj;
         r.eig_eps = s->params.eig_eps;
@@ -2336,7 +2298,7 @@ int enqueue_batch_frame(fvgs_batch* b, const Request* reqs, bool capture) {
                                       cudaMemcpyHostToDevice, b->stream));
             }
             FV_CK(launch_track_batch(jobs + (size_t)it * n, begin + (size_t)it * (n + 1), (int)n, total, b->tw[l],
-                                     b->th[l], b->analytic, b->variant[l], b->counters, b->num_sms, b->stream));
+                                     b->th[l], b->analytic, b->counters, b->num_sms, b->stream));
             FV_CK(launch_track_reduce_batch(rjobs + (size_t)it * n, (int)n, b->stream));
             b->batch_launches += 2;
             FV_TRY(batch_fork(b));
@@ -2431,7 +2393,7 @@ int batch_launch(fvgs_batch* b, const Request* reqs) {
             s->last_W = e.last_W;
             s->last_H = e.last_H;
             s->last_T = e.last_T;
-            s->last_split = 1;  // batched launches run one CTA per tile
+            s->last_split = e.last_split;
             s->keys_valid = false;
             s->has_binning = true;
             for (int c = 0; c < FVGS_K_COUNT; ++c) s->launches[c] += e.launches[c];
@@ -2492,6 +2454,7 @@ int batch_launch(fvgs_batch* b, const Request* reqs) {
         e.last_W = s->last_W;
         e.last_H = s->last_H;
         e.last_T = s->last_T;
+        e.last_split = s->last_split;
         for (int c = 0; c < FVGS_K_COUNT; ++c) e.launches[c] = s->launches[c] - before[i].launches[c];
     }
     fvgs_batch::Graph& g = b->graph;
@@ -2686,7 +2649,7 @@ int fvgs_batch_autotune(fvgs_batch* b, const fvgs_pose* poses, const fvgs_intrin
                 const int v = variants[vi];
                 for (int r = 0; r < reps && rc == FVGS_OK; ++r) {
                     if (cudaEventRecord(ev[2 * r], b->stream) != cudaSuccess ||
-                        launch_track_batch(b->d_jobs, b->d_begin, (int)n, total, b->tw[l], b->th[l], b->analytic, v,
+                        launch_track_batch(b->d_jobs, b->d_begin, (int)n, total, b->tw[l], b->th[l], b->analytic,
                                            b->counters, b->num_sms, b->stream) != cudaSuccess ||
                         cudaEventRecord(ev[2 * r + 1], b->stream) != cudaSuccess)
                         rc = FVGS_E_CUDA;
@@ -2698,8 +2661,13 @@ int fvgs_batch_autotune(fvgs_batch* b, const fvgs_pose* poses, const fvgs_intrin
                 std::sort(t.begin(), t.end());
                 const float med = t[reps / 2];
                 if (ms_out) ms_out[l * 9 + sh * 3 + vi] = med;
-                if (med < best) {
-                    best = med;
+                // A shape other than the reference's 16 x 16 has to be a quarter
+                // faster: it blends other lists (its own rectangles and
+                // tile-centre depths), and the launch timed here leaves out
+                // its binning (8 x 8 tiles list 2.5 times the instances).
+                const float cost = sh == 0 ? med : 1.25f * med;
+                if (cost < best) {
+                    best = cost;
                     best_shape = sh;
                     best_variant = v;
                 }

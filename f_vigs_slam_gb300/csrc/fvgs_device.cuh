@@ -181,17 +181,6 @@ __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// A Gaussian of opacity o yields alpha = min(0.99, o exp(-v/2)) < 1/255
-// (with or without the clamp) exactly when v > 2 ln(255 o).  The bound
-// returned is that value plus a margin far above the rounding of expf and of
-// the product, so pairs beyond it are rejected without evaluating the
-// exponential, with the same outcome.
-__device__ __forceinline__ float reject_bound(float o) {
-    if (!(o > 0.0f)) return -INFINITY;
-    const float b = 2.0f * logf(255.0f * o);
-    return b + 1e-3f + 1e-4f * fabsf(b);
-}
-
 // The conic's quadratic form v = a dx^2 + 2 b dx dy + c dy^2, evaluated as
 // dx * dl0 + dy * dl1 with dl0 = a dx + b dy, dl1 = b dx + c dy: the
 // gradient terms the backward passes need come for free.  A pass that
@@ -212,6 +201,16 @@ __device__ __forceinline__ float conic_form(float a, float b, float c, float dx,
 // NaN) opacity maps to -inf, i.e. weight 0: such a Gaussian never reaches
 // alpha 1/255, as o exp(-v/2) <= 0 never does.
 __device__ __forceinline__ float log2_opacity(float o) { return log2f(fmaxf(o, 0.0f)); }
+// A Gaussian of opacity o yields alpha = min(0.99, o exp(-v/2)) < 1/255
+// (with or without the clamp) exactly when v > 2 ln(255 o) = 2 ln 2 (log2 255 +
+// log2 o).  The bound returned is that value plus a margin far above the
+// rounding of the logarithm and of the weight, so pairs beyond it are
+// rejected without evaluating the exponential, with the same outcome.
+__device__ __forceinline__ float reject_bound(float o, float log2_o) {
+    if (!(o > 0.0f)) return -INFINITY;
+    const float b = 1.38629436f * (7.99435344f + log2_o);
+    return b + 1e-3f + 1e-4f * fabsf(b);
+}
 
 __device__ __forceinline__ float gauss_weight(float log2_o, float v) {
     float e;

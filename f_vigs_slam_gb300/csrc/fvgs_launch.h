@@ -4,7 +4,6 @@
 
 #include <cstddef>
 #include <cstdint>
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "../../include/fvgs_types.h"
@@ -94,11 +93,9 @@ struct ProjectArgs {
     float* dbg_cov;    // optional: 3N Sigma2D (xx, yy, xy)
     float* dbg_inv;    // optional: 3N inverse, stored order (xx, yy, xy)
     uint8_t* dbg_vis;  // optional: N visibility
-    // optional (analytic pose Jacobian): geometry record of every Gaussian
-    // with instances, geo0 = (Sxx, Sxy, Sxz, Syy), geo1 = (Syz, Szz, x, y) --
-    // the camera-frame 3D covariance and mean (z is rec0.z)
-    float4* geo0;
-    float4* geo1;
+    // optional (analytic pose Jacobian): the pose derivatives of every
+    // Gaussian with instances, 8 vectors each (pose_derivs)
+    float4* deriv;
     // optional candidate list (capacity n) and its state; cone: the current
     // view's largest angle from the optical axis (its farthest image corner),
     // radians -- a list built for a cone at least as wide is reused
@@ -240,18 +237,14 @@ struct TrackArgs {
     const float* ref_col;
     const float* ref_opa;
     uint32_t quirks;
-    // launch variant of the Jacobian kernel (the autotuner's choice): 0 = four
-    // CTAs per SM (64 registers), 1 = three CTAs per SM (80 registers), 2 =
-    // four CTAs per SM with the record batches gathered by TMA (needs the
-    // record tensor maps); the arithmetic and its order are the same in all
+    // launch variant of the Jacobian kernel (the autotuner's choice); the
+    // arithmetic and its order are the same in all
     int variant;
-    uint32_t* st_flags;  // status word for bounded-wait timeouts (variant 2)
-    // analytic pose Jacobian (FVGS_Q_POSE_JAC_APPROX clear): the geometry
-    // records written by the projection (ProjectArgs::geo0 / geo1)
-    const float4* geo0;
-    const float4* geo1;
+    // analytic pose Jacobian (FVGS_Q_POSE_JAC_APPROX clear): the derivatives
+    // written by the projection (ProjectArgs::deriv)
+    const float4* deriv;
     // tile shape of the binning the lists come from: 16 x 16 (also 0 x 0),
-    // 8 x 8 or 32 x 8 (the TMA-staged variant only for 16 x 16)
+    // 8 x 8 or 32 x 8
     int tile_w, tile_h;
     // precision form: compensated accumulation of the per-pixel colour
     // Jacobian and of the in-tile sums (analytic Jacobian, 16 x 16 tiles)
@@ -268,26 +261,21 @@ constexpr int kTrackVariants = 8;
 inline bool track_tile_supported(int tw, int th) {
     return (tw == 16 && th == 16) || (tw == 8 && th == 8) || (tw == 32 && th == 8);
 }
-// Gaussians staged per shared-memory batch by a launch variant: 3, 5, 6 ->
+// The staging batch that a batch's level reports (fvgs_batch_set_level): 3 ->
 // 128, 4 -> 512, otherwise 256.
-inline int track_variant_batch(int variant) {
-    return (variant == 3 || variant == 5 || variant == 6) ? 128 : (variant == 4 ? 512 : 256);
+inline int track_variant_batch(int variant) { return variant == 3 ? 128 : (variant == 4 ? 512 : 256); }
+// CTAs per 16 x 16 list tile of a launch variant: 4 (8 x 8 pixel quarters), 2
+// (16 x 8 halves) or 1.
+inline int track_variant_split(int variant) {
+    return (variant == 0 || variant == 3 || variant == 6) ? 4 : ((variant == 2 || variant == 4 || variant == 5) ? 2 : 1);
 }
-// CTAs per 16 x 16 list tile of a launch variant: 5 -> 2 (16 x 8 pixel
-// halves), 6 -> 4 (8 x 8 quarters), otherwise 1.  More, smaller CTAs fill
-// the SMs at the coarse pyramid levels, where a frame has a few hundred
-// tiles with long lists; every CTA stages its tile's whole list.
-inline int track_variant_split(int variant) { return variant == 5 ? 2 : (variant == 6 ? 4 : 1); }
+// The same for the persistent batched launch.
+inline int track_batch_split(int tw, int th) { return tw == 16 && th == 16 ? 4 : 1; }
 // Set the dynamic shared-memory limits of the tracking kernels on the current
-// device (their batches can exceed the 48 KB default); once per device,
+// device (their staging areas can exceed the 48 KB default); once per device,
 // before any launch or capture.
 cudaError_t track_configure_device();
-// Tensor maps of the three record planes (2-D: 4 floats x capacity rows,
-// 16-byte rows, one-row boxes) for the TMA-staged variant.
-struct RecMaps {
-    CUtensorMap rec[3];
-};
-cudaError_t launch_track(const TrackArgs& a, const RecMaps* maps, cudaStream_t s);
+cudaError_t launch_track(const TrackArgs& a, cudaStream_t s);
 // The tracking kernel reading the reference's separate screen-space buffers
 // instead of the packed record planes.
 cudaError_t launch_track_ref_layout(const TrackArgs& a, cudaStream_t s);
@@ -319,11 +307,12 @@ struct TrackJob {
 };
 // The tiles of n_jobs sessions in one persistent launch: work item i is tile
 // i - begin[j] of job j for begin[j] <= i < begin[j + 1] (begin: n_jobs + 1
-// device words).  Every job must use tile shape (tile_w, tile_h), the same
-// Jacobian mode (analytic) and staging batch (variant).  counters: two
+// device words; a 16 x 16 tile counts as track_batch_split items).  Every job
+// must use tile shape (tile_w, tile_h) and the same Jacobian mode (analytic).
+// counters: two
 // device words, zero before the first launch; every launch leaves them zero.
 cudaError_t launch_track_batch(const TrackJob* jobs, const uint32_t* begin, int n_jobs, uint32_t total_tiles,
-                               int tile_w, int tile_h, bool analytic, int variant, uint32_t* counters, int num_sms,
+                               int tile_w, int tile_h, bool analytic, uint32_t* counters, int num_sms,
                                cudaStream_t s);
 // Kernel attributes of the persistent kernels on the current device.
 cudaError_t track_batch_configure_device();

@@ -26,8 +26,19 @@
 //  * terms are accumulated in the camera frame (translation rows without R)
 //    and rotated once per frame, in FP64, by diag(R, I);
 //  * the 27 per-thread sums are reduced by a 31-shuffle butterfly
-//    reduce-scatter, then across the 8 warps in a fixed order, and written
-//    once per tile (no atomics: results are run-to-run deterministic).
+//    reduce-scatter, then across the CTA's warps in a fixed order, and written
+//    once per CTA (no atomics: results are run-to-run deterministic);
+//  * every warp stages and walks the list for its own 8 x 4 pixels
+//    (walk_list): no barrier before the CTA's final sum.
+//
+// What bounds it: instruction issue at the fine levels, latency at the coarse
+// ones.  On the 1 M room at 1280x720 the kernel with CTA-wide staging batches
+// took 401 / 155 / 92 us at levels 0 / 1 / 2 (its best launch form each); warps
+// that stage for themselves, with the pose derivatives computed once per
+// Gaussian by the projection instead of once per staged entry, take 350 / 125
+// / 62.  At level 2 the busiest SM sub-partition had executed twice the mean's
+// instructions (240 CTAs of 8 warps on 152 SMs) and a third of the stall was
+// the staging barriers.
 #include <cooperative_groups.h>
 
 #include "track_tile.cuh"
@@ -37,17 +48,12 @@ namespace cg = cooperative_groups;
 namespace fvgs {
 
 
-// The per-frame kernel: one CTA per tile of one session.
-template <int TW, int TH, bool RENDER_ONLY, bool REF_LAYOUT = false, int MIN_CTAS = 4, bool TMA = false,
-          int BATCH = kBatch, bool ANALYTIC = false, bool COMP = false>
-__global__ void __launch_bounds__(TW * TH, MIN_CTAS) track_tile_kernel(TrackArgs a, const __grid_constant__ RecMaps maps) {
+// The per-frame kernel: one CTA per tile (or part of a tile) of one session.
+template <int TW, int TH, bool RENDER_ONLY, bool REF_LAYOUT, int MIN_CTAS, bool ANALYTIC = false, bool COMP = false>
+__global__ void __launch_bounds__(TW * TH, MIN_CTAS) track_tile_kernel(TrackArgs a) {
     pdl_begin();
     extern __shared__ __align__(128) unsigned char s_dyn[];
-    if (TMA) {
-        if (threadIdx.x == 0) tma_bar_init(&body_tma_stage<TW, TH, BATCH, ANALYTIC>(s_dyn).bar);
-        __syncthreads();
-    }
-    track_tile_body<TW, TH, RENDER_ONLY, REF_LAYOUT, TMA, BATCH, ANALYTIC, COMP>(a, maps, blockIdx.x, s_dyn);
+    track_tile_body<TW, TH, RENDER_ONLY, REF_LAYOUT, ANALYTIC, COMP>(a, blockIdx.x, s_dyn);
 }
 
 // Cholesky of a symmetric 6x6 (lower factor in L); false if not positive
@@ -485,7 +491,7 @@ __global__ void __cluster_dims__(kRedCtas, 1, 1) __launch_bounds__(256)
 
 namespace {
 
-using TrackKernel = void (*)(TrackArgs, RecMaps);
+using TrackKernel = void (*)(TrackArgs);
 
 struct KernelPick {
     TrackKernel fn = nullptr;
@@ -493,67 +499,52 @@ struct KernelPick {
     size_t smem = 0;
 };
 
-template <int TW, int TH, bool RENDER_ONLY, bool REF_LAYOUT, int MIN_CTAS, bool TMA, int BATCH, bool ANALYTIC,
-          bool COMP = false>
+// REGS: the register budget per thread, as the CTAs per SM that it allows.
+// The default, 8 x 8 CTAs at the budget without spills inside the pair loop,
+// is the fastest or within 2% of it at every level measured (1 M room,
+// 1280x720, analytic, us at levels 0 / 1 / 2): 350 / 125 / 62, one CTA per
+// tile 365 / 131 / 70, at 96 registers 386 / 145 / 75, at 80 registers 407 / 154
+// / 88.  Small CTAs spread a coarse level's few tiles over all SMs, and a CTA
+// waits only for its own two blocks.
+template <int TW, int TH, bool RENDER_ONLY, int REGS, bool ANALYTIC, bool COMP = false>
 KernelPick pick() {
-    return {track_tile_kernel<TW, TH, RENDER_ONLY, REF_LAYOUT, MIN_CTAS, TMA, BATCH, ANALYTIC, COMP>, TW * TH,
-            body_smem_bytes<TW, TH, BATCH, ANALYTIC, TMA>()};
-}
-
-// Tiles of 8 x 8 and 32 x 8: the staging batch is the only launch choice;
-// MIN_CTAS gives the register budget of the 16 x 16 kernels' variant 1 for
-// the analytic Jacobian (80 per thread) and of variant 0 otherwise (64).
-template <int TW, int TH, bool ANALYTIC>
-KernelPick pick_shape(int variant) {
-    constexpr int M = (ANALYTIC ? 768 : 1024) / (TW * TH);
-    const int batch = track_variant_batch(variant);
-    if (batch == 128) return pick<TW, TH, false, false, M, false, 128, ANALYTIC>();
-    if (batch == 512) return pick<TW, TH, false, false, M, false, 512, ANALYTIC>();
-    return pick<TW, TH, false, false, M, false, 256, ANALYTIC>();
+    constexpr int M = (REGS == 64 ? 1024 : (REGS == 80 ? 768 : (REGS == 96 ? 640 : 512))) / (TW * TH);
+    return {track_tile_kernel<TW, TH, RENDER_ONLY, false, M, ANALYTIC, COMP>, TW * TH,
+            body_smem_bytes<TW, TH, ANALYTIC>()};
 }
 
 // The kernel of a tracking launch: tile shape, Jacobian mode and launch
 // variant (the autotuner's choice; the arithmetic and its order are the same
 // in all variants of a shape).
-KernelPick pick_track(const TrackArgs& a, bool have_maps) {
+template <bool ANALYTIC>
+KernelPick pick_jacobian(const TrackArgs& a, int tw, int th) {
+    constexpr int HIGH = ANALYTIC ? 128 : 96, MID = ANALYTIC ? 96 : 80, LOW = ANALYTIC ? 80 : 64;
+    if (tw == 8 && th == 8) return pick<8, 8, false, HIGH, ANALYTIC>();
+    if (tw == 32 && th == 8) return pick<32, 8, false, HIGH, ANALYTIC>();
+    if (tw != kTW || th != kTH) return {};
+    switch (a.variant) {
+        case 1: return pick<16, 16, false, HIGH, ANALYTIC>();
+        case 2: return pick<16, 8, false, HIGH, ANALYTIC>();
+        case 3: return pick<8, 8, false, MID, ANALYTIC>();
+        case 4: return pick<16, 8, false, MID, ANALYTIC>();
+        case 5: return pick<16, 8, false, LOW, ANALYTIC>();
+        case 6: return pick<8, 8, false, LOW, ANALYTIC>();
+        case 7: return pick<16, 16, false, LOW, ANALYTIC>();
+        default: return pick<8, 8, false, HIGH, ANALYTIC>();
+    }
+}
+
+KernelPick pick_track(const TrackArgs& a) {
     const bool analytic = !(a.quirks & FVGS_Q_POSE_JAC_APPROX);
     const int tw = a.tile_w ? a.tile_w : kTW, th = a.tile_h ? a.tile_h : kTH;
-    if (a.compensated && (!analytic || tw != kTW || th != kTH)) return {};
+    const bool tile16 = tw == kTW && th == kTH;
+    if (a.compensated && (!analytic || !tile16)) return {};
     const int split = a.split > 1 ? a.split : 1;
-    if (split > 1 && (a.compensated || a.render_only || tw != kTW || th != kTH)) return {};
-    if (a.render_only) {
-        if (tw != kTW || th != kTH) return {};
-        return pick<16, 16, true, false, 4, false, kBatch, false>();
-    }
-    if (tw == 8 && th == 8) return analytic ? pick_shape<8, 8, true>(a.variant) : pick_shape<8, 8, false>(a.variant);
-    if (tw == 32 && th == 8)
-        return analytic ? pick_shape<32, 8, true>(a.variant) : pick_shape<32, 8, false>(a.variant);
-    if (tw != kTW || th != kTH) return {};
-    if (analytic && a.compensated) return pick<16, 16, false, false, 3, false, 256, true, true>();
-    // 16 x 16 lists over 2 or 4 CTAs (the split matches the variant)
-    if (split != track_variant_split(a.variant)) return {};
-    if (a.variant == 5)
-        return analytic ? pick<16, 8, false, false, 6, false, 128, true>()
-                        : pick<16, 8, false, false, 8, false, 128, false>();
-    if (a.variant == 6)
-        return analytic ? pick<8, 8, false, false, 12, false, 128, true>()
-                        : pick<8, 8, false, false, 16, false, 128, false>();
-    if (analytic) {
-        // analytic Jacobian: plain staging (no TMA variant), one CTA per SM
-        // fewer than the reference Jacobian's variants (its fused pass holds
-        // the colour-Jacobian sums: 80 registers at three CTAs, 128 at two)
-        if (a.variant == 1) return pick<16, 16, false, false, 2, false, 256, true>();
-        if (a.variant == 7) return pick<16, 16, false, false, 2, false, 128, true>();
-        if (a.variant == 3) return pick<16, 16, false, false, 3, false, 128, true>();
-        if (a.variant == 4) return pick<16, 16, false, false, 3, false, 512, true>();
-        return pick<16, 16, false, false, 3, false, 256, true>();
-    }
-    if (a.variant == 1) return pick<16, 16, false, false, 3, false, 256, false>();
-    if (a.variant == 7) return pick<16, 16, false, false, 2, false, 256, false>();
-    if (a.variant == 3) return pick<16, 16, false, false, 4, false, 128, false>();
-    if (a.variant == 4) return pick<16, 16, false, false, 4, false, 512, false>();
-    if (a.variant == 2 && have_maps) return pick<16, 16, false, false, 4, true, 256, false>();
-    return pick<16, 16, false, false, 4, false, 256, false>();
+    if (split > 1 && (a.compensated || a.render_only || !tile16)) return {};
+    if (a.render_only) return tile16 ? pick<16, 16, true, 64, false>() : KernelPick{};
+    if (a.compensated) return pick<16, 16, false, 128, true, true>();
+    if (tile16 && split != track_variant_split(a.variant)) return {};
+    return analytic ? pick_jacobian<true>(a, tw, th) : pick_jacobian<false>(a, tw, th);
 }
 
 }  // namespace
@@ -572,39 +563,30 @@ cudaError_t track_configure_device() {
                     a.tile_h = shape == 0 ? 16 : 8;
                     a.variant = v % kTrackVariants;
                     if (shape == 0 && !a.compensated && !render) a.split = track_variant_split(a.variant);
-                    const KernelPick k = pick_track(a, true);
+                    const KernelPick k = pick_track(a);
                     if (!k.fn) continue;
                     const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k.fn),
                                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                                (int)k.smem);
                     if (e != cudaSuccess) return e;
                 }
-    const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(track_tile_kernel<16, 16, false, true>),
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)body_smem_bytes<16, 16, kBatch, false, false>());
-    if (e != cudaSuccess) return e;
     return track_batch_configure_device();
 }
 
-cudaError_t launch_track(const TrackArgs& a, const RecMaps* maps, cudaStream_t s) {
+cudaError_t launch_track(const TrackArgs& a, cudaStream_t s) {
     const int T = a.ntx * a.nty * (a.split > 1 ? a.split : 1);
     if (T <= 0) return cudaSuccess;
-    if (!a.render_only && !(a.quirks & FVGS_Q_POSE_JAC_APPROX) && (!a.geo0 || !a.geo1)) return cudaErrorInvalidValue;
-    if (a.variant == 2 && !a.render_only && (a.quirks & FVGS_Q_POSE_JAC_APPROX) &&
-        (a.tile_w == 0 || a.tile_w == kTW) && (a.tile_h == 0 || a.tile_h == kTH) && (!maps || !a.st_flags))
-        return cudaErrorInvalidValue;
-    const KernelPick k = pick_track(a, maps != nullptr);
+    if (!a.render_only && !(a.quirks & FVGS_Q_POSE_JAC_APPROX) && !a.deriv) return cudaErrorInvalidValue;
+    const KernelPick k = pick_track(a);
     if (!k.fn) return cudaErrorInvalidValue;
-    RecMaps m{};
-    if (maps) m = *maps;
-    return launch_chained(k.fn, dim3(T), dim3(k.threads), k.smem, s, a, m);
+    return launch_chained(k.fn, dim3(T), dim3(k.threads), k.smem, s, a);
 }
 
 cudaError_t launch_track_ref_layout(const TrackArgs& a, cudaStream_t s) {
     const int T = a.ntx * a.nty;
     if (T <= 0) return cudaSuccess;
-    return launch_chained(track_tile_kernel<16, 16, false, true>, dim3(T), dim3(kPix),
-                          body_smem_bytes<16, 16, kBatch, false, false>(), s, a, RecMaps{});
+    return launch_chained(track_tile_kernel<16, 16, false, true, 4>, dim3(T), dim3(kPix),
+                          body_smem_bytes<16, 16, false>(), s, a);
 }
 
 cudaError_t launch_track_reduce(const float* tile_out, int num_tiles, int split, DevPose* pose, double* out,

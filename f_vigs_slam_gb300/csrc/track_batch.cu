@@ -15,7 +15,7 @@
 
 namespace fvgs {
 
-template <int TW, int TH, int BATCH, bool ANALYTIC, int MIN_CTAS>
+template <int TW, int TH, bool ANALYTIC, int MIN_CTAS>
 __global__ void __launch_bounds__(TW * TH, MIN_CTAS)
     track_batch_kernel(const TrackJob* __restrict__ jobs, const uint32_t* __restrict__ begin, int n_jobs,
                        uint32_t total, uint32_t* counters) {
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(TW * TH, MIN_CTAS)
             __syncthreads();
             cur = job;
         }
-        track_tile_body<TW, TH, false, false, false, BATCH, ANALYTIC>(s_args, RecMaps{}, s_tile, s_dyn);
+        track_tile_body<TW, TH, false, false, ANALYTIC>(s_args, s_tile, s_dyn);
         __syncthreads();  // the tile's shared state is consumed before the next item is taken
     }
     // Every CTA that leaves has drawn an item past the end; the last one to
@@ -82,26 +82,18 @@ struct BatchPick {
     size_t smem = 0;
 };
 
-// Register budget: 64 per thread for the reference Jacobian, 80 for the
-// analytic one (its single fused pass holds the colour-Jacobian sums).
-template <int TW, int TH, int BATCH, bool ANALYTIC>
-BatchPick bpick() {
-    return {track_batch_kernel<TW, TH, BATCH, ANALYTIC, (ANALYTIC ? 768 : 1024) / (TW * TH)>, TW * TH,
-            body_smem_bytes<TW, TH, BATCH, ANALYTIC, false>()};
-}
-
+// Register budget: that of the per-frame kernel's default variant (128 per
+// thread for the analytic Jacobian, 96 for the reference's).
 template <int TW, int TH, bool ANALYTIC>
-BatchPick bpick_batch(int batch) {
-    if (batch == 128) return bpick<TW, TH, 128, ANALYTIC>();
-    if (batch == 512) return bpick<TW, TH, 512, ANALYTIC>();
-    return bpick<TW, TH, 256, ANALYTIC>();
+BatchPick bpick() {
+    return {track_batch_kernel<TW, TH, ANALYTIC, (ANALYTIC ? 512 : 640) / (TW * TH)>, TW * TH,
+            body_smem_bytes<TW, TH, ANALYTIC>()};
 }
 
-BatchPick pick_batch(int tw, int th, bool analytic, int variant) {
-    const int batch = track_variant_batch(variant);
-    if (tw == 16 && th == 16) return analytic ? bpick_batch<16, 16, true>(batch) : bpick_batch<16, 16, false>(batch);
-    if (tw == 8 && th == 8) return analytic ? bpick_batch<8, 8, true>(batch) : bpick_batch<8, 8, false>(batch);
-    if (tw == 32 && th == 8) return analytic ? bpick_batch<32, 8, true>(batch) : bpick_batch<32, 8, false>(batch);
+// A work item is a tile, or a quarter of a 16 x 16 tile (track_batch_split).
+BatchPick pick_batch(int tw, int th, bool analytic) {
+    if ((tw == 16 && th == 16) || (tw == 8 && th == 8)) return analytic ? bpick<8, 8, true>() : bpick<8, 8, false>();
+    if (tw == 32 && th == 8) return analytic ? bpick<32, 8, true>() : bpick<32, 8, false>();
     return {};
 }
 
@@ -132,23 +124,21 @@ int resident_blocks(const BatchPick& k) {
 
 cudaError_t track_batch_configure_device() {
     const int shapes[3][2] = {{16, 16}, {8, 8}, {32, 8}};
-    const int variants[3] = {0, 3, 4};  // batches of 256, 128, 512
     for (auto& sh : shapes)
-        for (int analytic = 0; analytic < 2; ++analytic)
-            for (int v : variants) {
-                const BatchPick k = pick_batch(sh[0], sh[1], analytic != 0, v);
-                const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k.fn),
-                                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
-                if (e != cudaSuccess) return e;
-            }
+        for (int analytic = 0; analytic < 2; ++analytic) {
+            const BatchPick k = pick_batch(sh[0], sh[1], analytic != 0);
+            const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k.fn),
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+            if (e != cudaSuccess) return e;
+        }
     return cudaSuccess;
 }
 
 cudaError_t launch_track_batch(const TrackJob* jobs, const uint32_t* begin, int n_jobs, uint32_t total_tiles,
-                               int tile_w, int tile_h, bool analytic, int variant, uint32_t* counters, int num_sms,
+                               int tile_w, int tile_h, bool analytic, uint32_t* counters, int num_sms,
                                cudaStream_t s) {
     if (n_jobs <= 0 || total_tiles == 0) return cudaSuccess;
-    const BatchPick k = pick_batch(tile_w, tile_h, analytic, variant);
+    const BatchPick k = pick_batch(tile_w, tile_h, analytic);
     if (!k.fn || !jobs || !begin || !counters) return cudaErrorInvalidValue;
     const uint32_t slots = (uint32_t)num_sms * (uint32_t)resident_blocks(k);
     const uint32_t grid = total_tiles < slots ? total_tiles : slots;

@@ -12,10 +12,9 @@
 
 namespace fvgs {
 
-// The default tile (16 x 16, one thread per pixel) -- the reference's TILE_SIZE
-// (src/GSCudaKernels.cu:6) -- and the only one of the TMA-staged variant.
+// The default tile (16 x 16, one thread per pixel): the reference's TILE_SIZE
+// (src/GSCudaKernels.cu:6).
 constexpr int kTW = 16, kTH = 16, kPix = kTW * kTH;
-constexpr int kBatch = 256;
 constexpr float kInv255 = 1.0f / 255.0f;
 
 // Error-free difference: hi + lo == a - b exactly (TwoSum).
@@ -131,457 +130,248 @@ __device__ __forceinline__ void warp_reduce_scatter32_comp(float (&v)[32], float
     lo = e[0];
 }
 
-// Stage one Gaussian's blending record: from the packed record planes, or
-// (REF_LAYOUT) built from the reference's separate screen-space buffers.
-template <bool REF_LAYOUT>
-__device__ __forceinline__ void load_record(const TrackArgs& a, uint32_t g, float4& r0, float4& r1, float4& r2) {
-    if (!REF_LAYOUT) {
-        r0 = a.rec0[g];
-        r1 = a.rec1[g];
-        r2 = a.rec2[g];
-    } else {
-        const float2 uv = reinterpret_cast<const float2*>(a.ref_uv)[g];
-        const float ixx = a.ref_inv[3 * (size_t)g], iyy = a.ref_inv[3 * (size_t)g + 1],
-                    ixy = a.ref_inv[3 * (size_t)g + 2];
-        const float2 ph = reinterpret_cast<const float2*>(a.ref_phat)[g];
-        const bool swap = (a.quirks & FVGS_Q_INVSIGMA_SWAP) != 0;
-        r0 = make_float4(uv.x, uv.y, a.ref_depth[g], a.ref_opa[g]);
-        r1 = make_float4(ixx, swap ? iyy : ixy, swap ? ixy : iyy, ph.x);
-        r2 = make_float4(ph.y, a.ref_col[3 * (size_t)g], a.ref_col[3 * (size_t)g + 1], a.ref_col[3 * (size_t)g + 2]);
-    }
+// One Gaussian's blending record built from the reference's separate
+// screen-space buffers.
+__device__ __forceinline__ void load_ref_record(const TrackArgs& a, uint32_t g, float4& r0, float4& r1, float4& r2) {
+    const float2 uv = reinterpret_cast<const float2*>(a.ref_uv)[g];
+    const float ixx = a.ref_inv[3 * (size_t)g], iyy = a.ref_inv[3 * (size_t)g + 1], ixy = a.ref_inv[3 * (size_t)g + 2];
+    const float2 ph = reinterpret_cast<const float2*>(a.ref_phat)[g];
+    const bool swap = (a.quirks & FVGS_Q_INVSIGMA_SWAP) != 0;
+    r0 = make_float4(uv.x, uv.y, a.ref_depth[g], a.ref_opa[g]);
+    r1 = make_float4(ixx, swap ? iyy : ixy, swap ? ixy : iyy, ph.x);
+    r2 = make_float4(ph.y, a.ref_col[3 * (size_t)g], a.ref_col[3 * (size_t)g + 1], a.ref_col[3 * (size_t)g + 2]);
 }
 
-// Minimum of q(dx, dy) = a dx^2 + 2 b dx dy + c dy^2 over the rectangle
-// [dxlo, dxhi] x [dylo, dyhi].  A positive definite q has its minimum at the
-// origin when the rectangle contains it; otherwise (and for any indefinite or
-// negative q) the minimum lies on the boundary, where each edge is a 1-D
-// quadratic: its endpoints, plus the clamped stationary point when convex.
-__device__ __forceinline__ float quad_min_rect(float a, float b, float c, float dxlo, float dxhi, float dylo,
-                                               float dyhi) {
-    if (a > 0.f && c > 0.f && a * c - b * b > 0.f && dxlo <= 0.f && dxhi >= 0.f && dylo <= 0.f && dyhi >= 0.f)
-        return 0.f;
-    float m = INFINITY;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const float X = e ? dxhi : dxlo;
-        const float Y = e ? dyhi : dylo;
-        // corners (each corner is visited once: (X, dylo), (X, dyhi))
-        m = fminf(m, a * X * X + 2.0f * b * X * dylo + c * dylo * dylo);
-        m = fminf(m, a * X * X + 2.0f * b * X * dyhi + c * dyhi * dyhi);
-        if (c > 0.f) {
-            const float dy = fminf(fmaxf(-b * X / c, dylo), dyhi);
-            m = fminf(m, a * X * X + 2.0f * b * X * dy + c * dy * dy);
-        }
-        if (a > 0.f) {
-            const float dx = fminf(fmaxf(-b * Y / a, dxlo), dxhi);
-            m = fminf(m, a * dx * dx + 2.0f * b * dx * Y + c * Y * Y);
-        }
-    }
-    return m;
-}
-
-// Tile-level rejection, done once per staged Gaussian.  A pixel skips a
-// Gaussian when v > vreject (alpha < 1/255, both passes) or, in the forward
-// pass only, when v <= 0.  If the extremes of v over the tile's pixel
-// rectangle prove one of these for every pixel -- min v > vreject, or (forward
-// pass) max v < 0 -- with a margin covering FP32 rounding at the magnitude of
-// the terms, the Gaussian is dropped from the staged batch.  Kept Gaussians
-// carry their original list index, so contributor counts and all results are
-// unchanged.  Non-finite records are always kept.
-template <bool FORWARD, int TW = kTW, int TH = kTH>
-__device__ __forceinline__ bool tile_prunable(float u, float v, float ca, float cb, float cc, float vrej, float x0,
-                                              float y0) {
-    if (vrej == -INFINITY) return true;  // zero opacity: alpha is 0 everywhere
-    if (!(isfinite(u) && isfinite(v) && isfinite(ca) && isfinite(cb) && isfinite(cc) && isfinite(vrej))) return false;
-    const float dxlo = u - (x0 + (float)(TW - 1)), dxhi = u - x0;
-    const float dylo = v - (y0 + (float)(TH - 1)), dyhi = v - y0;
+// Rejection of a Gaussian by a warp's 8 x 4 pixel block, once per staged
+// Gaussian.  A pixel skips a Gaussian when v > vreject (alpha < 1/255, both
+// passes) or, in the forward pass only, when v <= 0.  If the extremes of v
+// over the block prove one of these for every pixel -- kRejectAlpha: min v >
+// vreject, kRejectSign: max v < 0 -- with a margin covering FP32 rounding at
+// the magnitude of the terms, the Gaussian is dropped.  Kept Gaussians carry
+// their list index, so contributor counts and all results are unchanged.
+// Non-finite records are always kept.
+//
+// Positive definite forms (all of them unless the reference's swapped storage
+// of the inverse covariance is on) take a short way: v >= 0, and over a
+// rectangle without the mean the minimum lies on an edge that faces the mean
+// (the straight line from the minimum to the mean falls, so it leaves the
+// rectangle at once).  Those are the edge X = the rectangle's dx nearest to 0
+// and the edge Y = its dy nearest to 0; where such an edge does not face the
+// mean its candidate is still a point of the rectangle, so the smaller of the
+// two is the minimum.  Any other form has its extremes at the corners or, on
+// an edge, at the clamped stationary point of the 1-D quadratic there (a
+// minimum where it is convex, else a maximum).  The stationary points come
+// from rcp.approx: one ulp off changes v by 1e-14 of its terms.
+constexpr uint32_t kRejectAlpha = 1u, kRejectSign = 2u;
+__device__ __forceinline__ uint32_t block_reject(float u, float v, float ca, float cb, float cc, float vrej, float x0,
+                                                 float y0) {
+    if (vrej == -INFINITY) return kRejectAlpha;  // zero opacity: alpha is 0 everywhere
+    if (!(isfinite(u) && isfinite(v) && isfinite(ca) && isfinite(cb) && isfinite(cc) && isfinite(vrej))) return 0u;
+    const float dxlo = u - (x0 + 7.0f), dxhi = u - x0;
+    const float dylo = v - (y0 + 3.0f), dyhi = v - y0;
     const float mx = fmaxf(fabsf(dxlo), fabsf(dxhi)), my = fmaxf(fabsf(dylo), fabsf(dyhi));
     const float margin = 1e-5f * (fabsf(ca) * mx * mx + 2.0f * fabsf(cb) * mx * my + fabsf(cc) * my * my) + 1e-3f;
-    if (quad_min_rect(ca, cb, cc, dxlo, dxhi, dylo, dyhi) > vrej + margin) return true;
-    if (FORWARD && -quad_min_rect(-ca, -cb, -cc, dxlo, dxhi, dylo, dyhi) < -margin) return true;
-    return false;
-}
-
-// The warps of a TW x TH tile (8 x 4 pixel blocks, row-major) whose pixels a
-// staged Gaussian can reach: those whose block meets the axis-aligned box of
-// the ellipse v <= vreject (v = a dx^2 + 2 b dx dy + c dy^2, half-widths
-// sqrt(V c / det) and sqrt(V a / det)).  Every pixel outside it rejects the
-// Gaussian in both passes (v > vreject), so a warp whose block misses the box
-// may skip it without changing any result.  V = 1.05 vreject + 1e-3 and the
-// widths grow by 1% + 0.01 px: when det >= 1e-4 a c the FP32 evaluation of v
-// errs by less than 1.6% of v, so no pixel the kernel would keep falls
-// outside.  Forms that are not positive definite, nearly singular ones and
-// non-finite values reach every warp.
-template <int TW, int TH>
-__device__ __forceinline__ uint32_t warp_block_mask(float u, float v, float a, float b, float c, float vrej,
-                                                    float x0, float y0) {
-    constexpr int NW = TW * TH / 32, WX = TW / 8;
-    constexpr uint32_t kAll = (1u << NW) - 1u;
-    const float det = a * c - b * b;
-    const float vm = fmaf(vrej, 1.05f, 1e-3f);
-    if (!(a > 0.f && c > 0.f && det > 1e-4f * (a * c) && vm > 0.f && vm < INFINITY && isfinite(u) && isfinite(v)))
-        return kAll;
-    const float inv = __frcp_rn(det);
-    const float hx = fmaf(sqrtf(vm * c * inv), 1.01f, 0.01f), hy = fmaf(sqrtf(vm * a * inv), 1.01f, 0.01f);
-    if (!(hx < INFINITY && hy < INFINITY)) return kAll;
-    uint32_t m = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-        const float bx = x0 + (float)((w % WX) * 8), by = y0 + (float)((w / WX) * 4);
-        if (bx <= u + hx && bx + 7.0f >= u - hx && by <= v + hy && by + 3.0f >= v - hy) m |= 1u << w;
+    auto q = [&](float dx, float dy) { return ca * dx * dx + 2.0f * cb * dx * dy + cc * dy * dy; };
+    const float sy = -cb * rcp_approx(cc), sx = -cb * rcp_approx(ca);
+    auto on_x = [&](float X) { return q(X, fminf(fmaxf(sy * X, dylo), dyhi)); };
+    auto on_y = [&](float Y) { return q(fminf(fmaxf(sx * Y, dxlo), dxhi), Y); };
+    if (ca > 0.f && cc > 0.f && ca * cc - cb * cb > 0.f) {
+        const float X = fminf(fmaxf(0.f, dxlo), dxhi), Y = fminf(fmaxf(0.f, dylo), dyhi);
+        return fminf(on_x(X), on_y(Y)) > vrej + margin ? kRejectAlpha : 0u;
     }
-    return m;
+    const float q00 = q(dxlo, dylo), q01 = q(dxlo, dyhi), q10 = q(dxhi, dylo), q11 = q(dxhi, dyhi);
+    float lo = fminf(fminf(q00, q01), fminf(q10, q11)), hi = fmaxf(fmaxf(q00, q01), fmaxf(q10, q11));
+    // a form that is 0 in both squares has no stationary point on an edge
+    if (cc != 0.f) {
+        const float e0 = on_x(dxlo), e1 = on_x(dxhi);
+        lo = fminf(lo, fminf(e0, e1));
+        hi = fmaxf(hi, fmaxf(e0, e1));
+    }
+    if (ca != 0.f) {
+        const float e0 = on_y(dylo), e1 = on_y(dyhi);
+        lo = fminf(lo, fminf(e0, e1));
+        hi = fmaxf(hi, fmaxf(e0, e1));
+    }
+    return (lo > vrej + margin ? kRejectAlpha : 0u) | (hi < -margin ? kRejectSign : 0u);
 }
 
-// Shared-memory batch of Gaussians, repacked so a rejected pair needs two
-// loads: sA = (u, v, c.x, c.y), sB = (c.z, vreject, log2(opacity), z),
-// sC = (phat.x, phat.y, r, g), sD = b, s_orig = index in the tile's list;
-// for the Jacobian pass also NX planes sX: the reference Jacobian stages
-// sX[0] = (rgx, rgy, -fx rgx, -fy rgy), the mean's normalised ray and the
-// third row of the projection Jacobian without 1/d; the analytic Jacobian
-// stages eight planes with the derivatives of (u, v, a, b, c) with respect to
-// the camera-frame pose update and the mean's (x, y) (see stage_deriv).
-template <int BATCH = kBatch, int NX = 1, int NT = kPix>
-struct TrackBatch {
-    // wm[j]: the warps (8 x 4 pixel blocks) whose pixels staged Gaussian j
-    // can reach (warp_block_mask); bm[w][g]: bit k set when entry 32 g + k
-    // is in warp w's mask -- each warp walks only its own entries
-    uint8_t wm[BATCH];
-    uint32_t bm[NT / 32][BATCH / 32];
-    float4 A[BATCH];
-    float4 B[BATCH];
-    float4 C[BATCH];
-    float4 X[NX][BATCH];
-    float D[BATCH];
-    int orig[BATCH];
-    int wcnt[NT / 32];
+// One warp's staged Gaussians: the survivors of 32 list entries, repacked so a
+// rejected pair needs two loads: A = (u, v, c.x, c.y), B = (c.z, vreject,
+// log2(opacity), z), C = (phat.x, phat.y, r, g), E = (b, list index), G =
+// Gaussian index; for the Jacobians also X: the reference Jacobian stages
+// X[j][0] = (rgx, rgy, -fx rgx, -fy rgy), the mean's normalised ray and the
+// third row of the projection Jacobian without 1/d; the analytic Jacobian the
+// eight vectors of pose_derivs.  An odd count is filled up with an entry that
+// every pixel rejects, so the entries are taken in pairs.
+constexpr int kRound = 32;  // list entries a warp stages at a time
+constexpr int kMaskRounds = 32;
+template <int NX>
+struct WarpStage {
+    float4 A[kRound];
+    float4 B[kRound];
+    float4 C[kRound];
+    float4 X[NX ? kRound : 1][NX ? NX : 1];
+    float2 E[kRound];
+    uint32_t G[kRound];
+    float4 R[3][kRound];  // the next round's records, each lane its own entry
+    uint32_t M[kMaskRounds];  // reference Jacobian: the second pass's survivors of each round
 };
 
 // What a staging round stores besides the blending record.
 enum StageExtra { kStageNone = 0, kStageRay = 1, kStageDeriv = 2 };
 
-// Derivatives of one Gaussian's screen mean (u, v) and consumed conic slots
-// (a, b, c) with respect to the camera-frame pose update delta = (dp_c,
-// dtheta): t' = t + R dp_c, R' = R exp(dtheta), so d p_cam / d dp_c = -I,
-// d p_cam / d dtheta = [p_cam]x and d Sigma_cam / d dtheta_j =
-// -[e_j]x Sigma_cam + Sigma_cam [e_j]x.  With J the projection's Jacobian
-// (rows J0, J1), M = Sigma_cam J^T and Q = Sigma2D^-1:
-//   d Sigma2D = dJ M + (dJ M)^T (+ the rotated-covariance terms
-//   2 J0 x M0, J0 x M1 + J1 x M0, 2 J1 x M1 for dtheta), dQ = -Q dSigma2D Q.
-// r0, r1: the blending record; g0, g1: the geometry record (camera-frame
-// covariance and mean).  out: du, dv, da, db, dc grouped by pairs of pose
-// coordinates (2m, 2m + 1), each quantity's pair adjacent (the order the
-// fused pass reads them in, deriv_pairs), then the mean's x, y.
-__device__ __forceinline__ void stage_deriv(const TrackArgs& a, const float4& r0, const float4& r1, const float4& g0,
-                                            const float4& g1, float4 (&out)[8]) {
-    const bool swap = (a.quirks & FVGS_Q_INVSIGMA_SWAP) != 0;
-    const float fx = a.K.fx, fy = a.K.fy;
-    const float z = r0.z, x = g1.z, y = g1.w;
-    const float sxx = g0.x, sxy = g0.y, sxz = g0.z, syy = g0.w, syz = g1.x, szz = g1.y;
-    const float q00 = r1.x, q01 = swap ? r1.z : r1.y, q11 = swap ? r1.y : r1.z;
-    const float iz = __frcp_rn(z), iz2 = iz * iz, iz3 = iz2 * iz;
-    // J0 = (j00, 0, j02), J1 = (0, j11, j12)
-    const float j00 = fx * iz, j02 = -fx * x * iz2, j11 = fy * iz, j12 = -fy * y * iz2;
-    const float m0x = sxx * j00 + sxz * j02, m0y = sxy * j00 + syz * j02, m0z = sxz * j00 + szz * j02;
-    const float m1x = sxy * j11 + sxz * j12, m1y = syy * j11 + syz * j12, m1z = syz * j11 + szz * j12;
-    // rotated-covariance terms: w00 = 2 J0 x M0, w01 = J0 x M1 + J1 x M0, w11 = 2 J1 x M1
-    const float w00[3] = {2.f * (-j02 * m0y), 2.f * (j02 * m0x - j00 * m0z), 2.f * (j00 * m0y)};
-    const float w01[3] = {-j02 * m1y + (j11 * m0z - j12 * m0y), (j02 * m1x - j00 * m1z) + j12 * m0x,
-                          j00 * m1y - j11 * m0x};
-    const float w11[3] = {2.f * (j11 * m1z - j12 * m1y), 2.f * (j12 * m1x), 2.f * (-j11 * m1x)};
-    const float qa = q00 * q00, qb = 2.f * q00 * q01, qc = q01 * q01;
-    const float qd = q00 * q01, qe = q00 * q11 + q01 * q01, qf = q01 * q11;
-    const float qg = 2.f * q01 * q11, qh = q11 * q11;
-    float du[6], dv[6], da[6], db[6], dc[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        // d p_cam for tangent direction k
-        const float dpx = k == 0 ? -1.f : (k == 4 ? -z : (k == 5 ? y : 0.f));
-        const float dpy = k == 1 ? -1.f : (k == 3 ? z : (k == 5 ? -x : 0.f));
-        const float dpz = k == 2 ? -1.f : (k == 3 ? -y : (k == 4 ? x : 0.f));
-        const float dj00 = -fx * iz2 * dpz;
-        const float dj02 = -fx * iz2 * dpx + 2.f * fx * x * iz3 * dpz;
-        const float dj11 = -fy * iz2 * dpz;
-        const float dj12 = -fy * iz2 * dpy + 2.f * fy * y * iz3 * dpz;
-        float ds00 = 2.f * (dj00 * m0x + dj02 * m0z);
-        float ds01 = (dj00 * m1x + dj02 * m1z) + (dj11 * m0y + dj12 * m0z);
-        float ds11 = 2.f * (dj11 * m1y + dj12 * m1z);
-        if (k >= 3) {
-            ds00 += w00[k - 3];
-            ds01 += w01[k - 3];
-            ds11 += w11[k - 3];
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// Walk the first n entries of the tile's list for one warp's 8 x 4 pixel
+// block with corner (x0, y0), front to back, until every lane is done.  The
+// warp stages kRound entries at a time on its own -- each lane takes one
+// entry, drops it when the block cannot see it, and the survivors are
+// compacted in list order -- so no barrier ties it to the tile's other warps:
+// a warp stops as soon as its own 32 pixels are opaque, and the tile's slowest
+// block delays nobody.  The next round's records are loaded while this
+// one's are blended.  pair(j, A, B, dx, dy, dl0, dl1, v, raw): one staged
+// Gaussian for every lane; round_end(): after each round.
+// MASKS: this walk's use of the kept survivors of the second pass (the
+// reference Jacobian's rejection test costs more than the rest of its staging,
+// and the first pass has both answers at hand).
+enum WalkMasks { kMasksNone = 0, kMasksKeep = 1, kMasksUse = 2 };
+template <bool REF_LAYOUT, int MASKS, int STAGE, int NX, class Pair, class RoundEnd>
+__device__ __forceinline__ void walk_list(const TrackArgs& a, WarpStage<NX>& ws, uint32_t list0, int n, float x0,
+                                          float y0, float xf, float yf, bool& done, Pair&& pair,
+                                          RoundEnd&& round_end) {
+    const int lane = threadIdx.x & 31;
+    if (__all_sync(kFullMask, done)) return;
+    __syncwarp();  // the staging area may still be read from an earlier walk
+    // the packed records travel to shared memory while the round before is
+    // blended (in registers they would be spilled around the pair loop)
+    auto fetch = [&](uint32_t gi) {
+        if constexpr (!REF_LAYOUT) {
+            if (gi < a.n_gauss) {
+                cp_async16(&ws.R[0][lane], a.rec0 + gi);
+                cp_async16(&ws.R[1][lane], a.rec1 + gi);
+                cp_async16(&ws.R[2][lane], a.rec2 + gi);
+            }
+            cp_async_commit();
         }
-        const float dq00 = -(qa * ds00 + qb * ds01 + qc * ds11);
-        const float dq01 = -(qd * ds00 + qe * ds01 + qf * ds11);
-        const float dq11 = -(qc * ds00 + qg * ds01 + qh * ds11);
-        du[k] = j00 * dpx + j02 * dpz;
-        dv[k] = j11 * dpy + j12 * dpz;
-        da[k] = dq00;
-        db[k] = swap ? dq11 : dq01;
-        dc[k] = swap ? dq01 : dq11;
+    };
+    uint32_t g = lane < n ? a.indices[list0 + lane] : 0xffffffffu;
+    fetch(g);
+    for (int base = 0; base < n; base += kRound) {
+        const int li = base + lane;
+        const uint32_t g_next = li + kRound < n ? a.indices[list0 + li + kRound] : 0xffffffffu;
+        bool keep = false;
+        uint32_t rej = kRejectAlpha;
+        float vrej = 0.f, lo2 = 0.f;
+        float4 r0, r1, r2;
+        if constexpr (!REF_LAYOUT) cp_async_wait<0>();
+        if (g < a.n_gauss) {
+            if constexpr (REF_LAYOUT) {
+                load_ref_record(a, g, r0, r1, r2);
+            } else {
+                r0 = ws.R[0][lane];
+                r1 = ws.R[1][lane];
+                r2 = ws.R[2][lane];
+            }
+            lo2 = log2_opacity(r0.w);
+            vrej = reject_bound(r0.w, lo2);
+            if (MASKS == kMasksUse && base < kRound * kMaskRounds)
+                keep = (ws.M[base / kRound] >> lane) & 1u;
+            else {
+                rej = block_reject(r0.x, r0.y, r1.x, r1.y, r1.z, vrej, x0, y0);
+                keep = MASKS == kMasksUse ? !(rej & kRejectAlpha) : rej == 0u;
+            }
+        }
+        if constexpr (MASKS == kMasksKeep) {
+            const uint32_t m = __ballot_sync(kFullMask, !(rej & kRejectAlpha));
+            if (lane == 0 && base < kRound * kMaskRounds) ws.M[base / kRound] = m;
+        }
+        const uint32_t bal = __ballot_sync(kFullMask, keep);
+        const int cnt = __popc(bal);
+        if (keep) {
+            const int pos = __popc(bal & lanemask_lt());
+            ws.A[pos] = make_float4(r0.x, r0.y, r1.x, r1.y);
+            ws.B[pos] = make_float4(r1.z, vrej, lo2, r0.z);
+            ws.C[pos] = make_float4(r1.w, r2.x, r2.y, r2.z);
+            ws.E[pos] = make_float2(r2.w, __int_as_float(li));
+            if constexpr (STAGE == kStageDeriv) ws.G[pos] = g;
+            if constexpr (STAGE == kStageRay) {
+                const float rgx = (r0.x - a.K.cx) * __frcp_rn(a.K.fx), rgy = (r0.y - a.K.cy) * __frcp_rn(a.K.fy);
+                ws.X[pos][0] = make_float4(rgx, rgy, -a.K.fx * rgx, -a.K.fy * rgy);
+            }
+        }
+        if (lane == 0 && (cnt & 1)) {
+            ws.A[cnt] = make_float4(0.f, 0.f, 0.f, 0.f);
+            ws.B[cnt] = make_float4(0.f, -INFINITY, -INFINITY, 0.f);
+        }
+        __syncwarp();
+        if constexpr (STAGE == kStageDeriv) {
+            // eight lanes bring one survivor's 128 bytes
+            static_assert(NX == 8, "the analytic Jacobian stages eight derivative vectors");
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int slot = 4 * k + (lane >> 3);
+                if (slot < cnt) cp_async16(&ws.X[slot][lane & 7], a.deriv + 8 * (size_t)ws.G[slot] + (lane & 7));
+            }
+            cp_async_commit();
+        }
+        g = g_next;
+        fetch(g);
+        if constexpr (STAGE == kStageDeriv) {
+            cp_async_wait<1>();  // the derivatives; the records stay in flight
+            __syncwarp();
+        }
+        // two entries per step: both quadratic forms and weights are
+        // evaluated before the branches, in list order
+        for (int j = 0; j < cnt; j += 2) {
+            const float4 A0 = ws.A[j], A1 = ws.A[j + 1];
+            const float4 B0 = ws.B[j], B1 = ws.B[j + 1];
+            const float dx0 = A0.x - xf, dy0 = A0.y - yf, dx1 = A1.x - xf, dy1 = A1.y - yf;
+            float l00, l01, l10, l11;
+            const float v0 = conic_form(A0.z, A0.w, B0.x, dx0, dy0, l00, l01);
+            const float v1 = conic_form(A1.z, A1.w, B1.x, dx1, dy1, l10, l11);
+            const float w0 = gauss_weight(B0.z, v0), w1 = gauss_weight(B1.z, v1);
+            pair(j, A0, B0, dx0, dy0, l00, l01, v0, w0);
+            pair(j + 1, A1, B1, dx1, dy1, l10, l11, v1, w1);
+            if (__all_sync(kFullMask, done)) break;
+        }
+        round_end();
+        if (__all_sync(kFullMask, done)) break;
+        __syncwarp();  // every lane is through with the staged entries
     }
-    out[0] = make_float4(du[0], du[1], dv[0], dv[1]);
-    out[1] = make_float4(da[0], da[1], db[0], db[1]);
-    out[2] = make_float4(dc[0], dc[1], du[2], du[3]);
-    out[3] = make_float4(dv[2], dv[3], da[2], da[3]);
-    out[4] = make_float4(db[2], db[3], dc[2], dc[3]);
-    out[5] = make_float4(du[4], du[5], dv[4], dv[5]);
-    out[6] = make_float4(da[4], da[5], db[4], db[5]);
-    out[7] = make_float4(dc[4], dc[5], x, y);
+    if constexpr (!REF_LAYOUT) cp_async_wait<0>();
 }
 
 // The derivatives of pose-coordinate pair m (2m, 2m + 1) of staged Gaussian
-// j (stage_deriv's layout): du, dv, da, db, dc as float2 (register pairs).
+// j (pose_derivs' layout): du, dv, da, db, dc as float2 (register pairs).
 struct DerivPair {
     float2 du, dv, da, db, dc;
 };
 // One pair at a time (three or two 16-byte and one 8-byte shared load), so
 // the fused pass holds one pair's ten values rather than all thirty.
-template <int BATCH, int NX>
-__device__ __forceinline__ DerivPair deriv_pair(const float4 (&X)[NX][BATCH], int j, int m) {
-    auto lo = [&](int plane) { return *reinterpret_cast<const float2*>(&X[plane][j].x); };
-    auto hi = [&](int plane) { return *reinterpret_cast<const float2*>(&X[plane][j].z); };
+__device__ __forceinline__ DerivPair deriv_pair(const float4 (&X)[8], int m) {
+    auto lo = [&](int plane) { return *reinterpret_cast<const float2*>(&X[plane].x); };
+    auto hi = [&](int plane) { return *reinterpret_cast<const float2*>(&X[plane].z); };
     if (m == 0) {
-        const float4 p0 = X[0][j], p1 = X[1][j];
+        const float4 p0 = X[0], p1 = X[1];
         return {make_float2(p0.x, p0.y), make_float2(p0.z, p0.w), make_float2(p1.x, p1.y), make_float2(p1.z, p1.w),
                 lo(2)};
     }
     if (m == 1) {
-        const float4 p3 = X[3][j], p4 = X[4][j];
+        const float4 p3 = X[3], p4 = X[4];
         return {hi(2), make_float2(p3.x, p3.y), make_float2(p3.z, p3.w), make_float2(p4.x, p4.y),
                 make_float2(p4.z, p4.w)};
     }
-    const float4 p5 = X[5][j], p6 = X[6][j];
+    const float4 p5 = X[5], p6 = X[6];
     return {make_float2(p5.x, p5.y), make_float2(p5.z, p5.w), make_float2(p6.x, p6.y), make_float2(p6.z, p6.w),
             lo(7)};
-}
-
-template <int STAGE, int TW, int TH, int BATCH, int NX, int NT>
-__device__ __forceinline__ void put_staged(const TrackArgs& a, TrackBatch<BATCH, NX, NT>& sb, int pos, const float4& r0,
-                                           const float4& r1, const float4& r2, float vrej, int li, uint32_t g,
-                                           float x0, float y0) {
-    static_assert(TW * TH == NT, "tile shape of the staged batch");
-    sb.wm[pos] = (uint8_t)warp_block_mask<TW, TH>(r0.x, r0.y, r1.x, r1.y, r1.z, vrej, x0, y0);
-    sb.A[pos] = make_float4(r0.x, r0.y, r1.x, r1.y);
-    sb.B[pos] = make_float4(r1.z, vrej, log2_opacity(r0.w), r0.z);
-    sb.C[pos] = make_float4(r1.w, r2.x, r2.y, r2.z);
-    sb.D[pos] = r2.w;
-    sb.orig[pos] = li;
-    if constexpr (STAGE == kStageRay) {
-        const float rgx = (r0.x - a.K.cx) * __frcp_rn(a.K.fx), rgy = (r0.y - a.K.cy) * __frcp_rn(a.K.fy);
-        sb.X[0][pos] = make_float4(rgx, rgy, -a.K.fx * rgx, -a.K.fy * rgy);
-    } else if constexpr (STAGE == kStageDeriv) {
-        static_assert(NX == 8, "the analytic Jacobian stages eight derivative planes");
-        float4 d[8];
-        stage_deriv(a, r0, r1, a.geo0[g], a.geo1[g], d);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) sb.X[k][pos] = d[k];
-    }
-}
-
-// Stage entries [base, min(base+BATCH, limit)) of the tile's list, dropping
-// the ones tile_prunable rejects; returns the number kept.  The CTA takes the
-// entries TW * TH at a time (one per thread; a smaller BATCH uses part of them),
-// each round compacted after the previous one, so the staged order is the
-// list order.  Ends with a barrier.
-template <bool REF_LAYOUT, bool FORWARD, int STAGE, int TW, int TH, int BATCH, int NX>
-__device__ __forceinline__ int stage_batch(const TrackArgs& a, TrackBatch<BATCH, NX, TW * TH>& sb, uint32_t list0, int base,
-                                           int limit, float x0, float y0) {
-    constexpr int NT = TW * TH;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    int total = 0;
-#pragma unroll
-    for (int r0 = 0; r0 < BATCH; r0 += NT) {
-        const int li = base + r0 + tid;
-        bool keep = false;
-        float4 r0v, r1, r2;
-        float vrej = 0.f;
-        uint32_t g = 0;
-        if (r0 + tid < BATCH && li < limit) {
-            g = a.indices[list0 + li];
-            if (g < a.n_gauss) {
-                load_record<REF_LAYOUT>(a, g, r0v, r1, r2);
-                vrej = reject_bound(r0v.w);
-                keep = !tile_prunable<FORWARD, TW, TH>(r0v.x, r0v.y, r1.x, r1.y, r1.z, vrej, x0, y0);
-            }
-        }
-        const uint32_t bal = __ballot_sync(kFullMask, keep);
-        if (lane == 0) sb.wcnt[w] = __popc(bal);
-        __syncthreads();
-        int wbase = 0, round_total = 0;
-#pragma unroll
-        for (int k = 0; k < NT / 32; ++k) {
-            const int c = sb.wcnt[k];
-            wbase += (k < w) ? c : 0;
-            round_total += c;
-        }
-        if (keep)
-            put_staged<STAGE, TW, TH>(a, sb, total + wbase + __popc(bal & lanemask_lt()), r0v, r1, r2, vrej, li, g,
-                                      x0, y0);
-        total += round_total;
-        __syncthreads();
-    }
-    return total;
-}
-
-// ---------------------------------------------------------------------------
-// TMA staging (launch variant 2).  The records of a batch are gathered into
-// shared memory by tile::gather4 tensor copies -- four Gaussians' 16-byte rows
-// of one record plane per copy, 192 copies per batch -- completing on an
-// mbarrier.  The next batch is gathered while the current one is blended, so
-// the records' load latency leaves the blending warps.  The staging itself
-// (rejection test, compaction into TrackBatch) is the same as stage_batch's.
-// Row indices outside the map (past the list, or defensive out-of-range
-// values) are replaced by row 0 and the row is not staged, so every copy
-// reads inside the record planes and transfers exactly 64 bytes.
-constexpr int kGroups = kBatch / 4;
-constexpr uint32_t kTmaBatchBytes = 3u * kGroups * 64u;
-
-struct TmaStage {
-    float4 raw[3][kGroups][8];  // plane, group of 4 Gaussians (128-byte slots, first 64 bytes used)
-    uint32_t gid[kBatch];       // the batch's Gaussian indices (0xffffffff past the list)
-    unsigned long long bar;
-};
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void tma_bar_init(unsigned long long* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void tma_bar_expect(unsigned long long* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
-// Bounded wait for the completion of the phase with the given parity.
-__device__ __forceinline__ bool tma_bar_wait(unsigned long long* bar, uint32_t parity) {
-    uint32_t done = 0;
-    for (uint32_t it = 0; it < kSpinLimit && !done; ++it)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-    return done != 0;
-}
-
-__device__ __forceinline__ void tma_gather4(float4* dst, const CUtensorMap* map, uint32_t r0, uint32_t r1,
-                                            uint32_t r2, uint32_t r3, unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Issue the gathers of entries [base, base + kBatch) of the tile's list (the
-// expected bytes were announced before the preceding barrier).
-__device__ __forceinline__ void tma_issue(const TrackArgs& a, const RecMaps& maps, TmaStage& ts, uint32_t list0,
-                                          int base, int limit) {
-    const int tid = threadIdx.x;
-    {
-        const int li = base + tid;
-        ts.gid[tid] = li < limit ? a.indices[list0 + li] : 0xffffffffu;
-    }
-    if (tid < 3 * kGroups) {
-        // the rows of the previous batch were read through the generic proxy
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const int plane = tid / kGroups, grp = tid % kGroups;
-        uint32_t r[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int li = base + 4 * grp + j;
-            const uint32_t g = li < limit ? a.indices[list0 + li] : 0u;
-            r[j] = g < a.n_gauss ? g : 0u;
-        }
-        tma_gather4(&ts.raw[plane][grp][0], &maps.rec[plane], r[0], r[1], r[2], r[3], &ts.bar);
-    }
-}
-
-// stage_batch with the records taken from the gathered batch; also announces
-// and issues the gathers of the next batch once this one is consumed.
-// parity / pending / broken track the mbarrier (uniform across the CTA).  A
-// wait that gives up flags kErrTimeout and leaves the copy pending: nothing
-// more is staged or issued, and the end of the pass waits for it once more.
-struct TmaState {
-    uint32_t parity = 0;
-    bool pending = false;
-    bool broken = false;
-};
-
-template <bool FORWARD>
-__device__ __forceinline__ int stage_batch_tma(const TrackArgs& a, const RecMaps& maps, TrackBatch<>& sb, TmaStage& ts,
-                                               uint32_t list0, int base, int limit, float x0, float y0,
-                                               TmaState& tm) {
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    bool ready = !tm.broken;
-    if (ready && tm.pending) {
-        ready = tma_bar_wait(&ts.bar, tm.parity);
-        if (ready) {
-            tm.parity ^= 1u;
-            tm.pending = false;
-        } else {
-            tm.broken = true;
-            if (tid == 0) atomicOr(&a.st_flags[0], kErrTimeout);
-        }
-    }
-    const int li = base + tid;
-    bool keep = false;
-    float4 r0, r1, r2;
-    float vrej = 0.f;
-    const uint32_t g = ts.gid[tid];
-    if (ready && li < limit && g < a.n_gauss) {
-        r0 = ts.raw[0][tid >> 2][tid & 3];
-        r1 = ts.raw[1][tid >> 2][tid & 3];
-        r2 = ts.raw[2][tid >> 2][tid & 3];
-        vrej = reject_bound(r0.w);
-        keep = !tile_prunable<FORWARD>(r0.x, r0.y, r1.x, r1.y, r1.z, vrej, x0, y0);
-    }
-    const uint32_t bal = __ballot_sync(kFullMask, keep);
-    if (lane == 0) sb.wcnt[w] = __popc(bal);
-    __syncthreads();  // the batch's raw rows and indices are consumed
-    int wbase = 0, total = 0;
-#pragma unroll
-    for (int k = 0; k < kPix / 32; ++k) {
-        const int c = sb.wcnt[k];
-        wbase += (k < w) ? c : 0;
-        total += c;
-    }
-    if (keep)
-        put_staged<FORWARD ? kStageNone : kStageRay, kTW, kTH>(a, sb, wbase + __popc(bal & lanemask_lt()), r0, r1, r2,
-                                                             vrej, li, g, x0, y0);
-    const bool next = ready && base + kBatch < limit;
-    if (next && tid == 0) tma_bar_expect(&ts.bar, kTmaBatchBytes);
-    __syncthreads();
-    if (next) {
-        tma_issue(a, maps, ts, list0, base + kBatch, limit);
-        tm.pending = true;
-    }
-    return total;
-}
-
-// Start a pass: announce and gather its first batch.
-__device__ __forceinline__ void tma_begin(const TrackArgs& a, const RecMaps& maps, TmaStage& ts, uint32_t list0,
-                                          int limit, TmaState& tm) {
-    if (limit <= 0 || tm.broken) return;
-    if (threadIdx.x == 0) tma_bar_expect(&ts.bar, kTmaBatchBytes);
-    __syncthreads();
-    tma_issue(a, maps, ts, list0, 0, limit);
-    tm.pending = true;
-}
-
-// End a pass: wait (bounded) for a gather still in flight, since the buffer
-// is reused or the CTA exits.
-__device__ __forceinline__ void tma_drain(const TrackArgs& a, TmaStage& ts, TmaState& tm) {
-    if (!tm.pending) return;
-    if (tma_bar_wait(&ts.bar, tm.parity)) {
-        tm.parity ^= 1u;
-        tm.pending = false;
-    } else {
-        tm.broken = true;
-        if (threadIdx.x == 0) atomicOr(&a.st_flags[0], kErrTimeout);
-    }
 }
 
 // Depth weight of a pixel's depth residual: the reference's
@@ -600,36 +390,12 @@ __device__ __forceinline__ float depth_weight(float derr, float thr, float z_obs
     return w / z_obs;
 }
 
-// Per-warp bitmaps of a staged batch of cnt entries (after its barrier; every
-// lane of the CTA takes part).  A warp writes and reads only its own rows.
-template <int BATCH, int NX, int NT>
-__device__ __forceinline__ void build_warp_bitmaps(TrackBatch<BATCH, NX, NT>& sb, int cnt) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int g = 0; g * 32 < cnt; ++g) {
-        const int j = g * 32 + lane;
-        const bool rel = j < cnt && ((sb.wm[j] >> w) & 1u);
-        const uint32_t b = __ballot_sync(kFullMask, rel);
-        if (lane == 0) sb.bm[w][g] = b;
-    }
-    __syncwarp();
-}
-
-// Shared-memory batch of the body below (dynamic shared memory: the analytic
-// Jacobian's batch of 512 exceeds the static limit).
-template <int TW, int TH, int BATCH, bool ANALYTIC>
-using BodyBatch = TrackBatch<BATCH, ANALYTIC ? 8 : 1, TW * TH>;
-
-// Dynamic shared memory of one CTA running the body: the staged batch, then
-// (TMA variant) the gathered batch at a 128-byte boundary.
-template <int TW, int TH, int BATCH, bool ANALYTIC, bool TMA>
+// Dynamic shared memory of one CTA running the body: a staging area per warp.
+template <int TW, int TH, bool ANALYTIC>
+using BodyStage = WarpStage<ANALYTIC ? 8 : 1>;
+template <int TW, int TH, bool ANALYTIC>
 constexpr size_t body_smem_bytes() {
-    return sizeof(BodyBatch<TW, TH, BATCH, ANALYTIC>) + (TMA ? sizeof(TmaStage) + 128 : 0);
-}
-
-template <int TW, int TH, int BATCH, bool ANALYTIC>
-__device__ __forceinline__ TmaStage& body_tma_stage(unsigned char* dyn) {
-    const uintptr_t p = reinterpret_cast<uintptr_t>(dyn) + sizeof(BodyBatch<TW, TH, BATCH, ANALYTIC>);
-    return *reinterpret_cast<TmaStage*>((p + 127) & ~uintptr_t(127));
+    return sizeof(BodyStage<TW, TH, ANALYTIC>) * (TW * TH / 32);
 }
 
 // One tile of the fused tracking kernel, run by a CTA of TW * TH threads (one
@@ -668,24 +434,17 @@ __device__ __forceinline__ float cta_partial_sum(const float (*s_red)[32], int c
     }
 }
 
-template <int TW, int TH, bool RENDER_ONLY, bool REF_LAYOUT, bool TMA, int BATCH, bool ANALYTIC,
-          bool COMP = false>
-__device__ __forceinline__ void track_tile_body(const TrackArgs& a, const RecMaps& maps, int tile,
-                                                unsigned char* dyn) {
+template <int TW, int TH, bool RENDER_ONLY, bool REF_LAYOUT, bool ANALYTIC, bool COMP = false>
+__device__ __forceinline__ void track_tile_body(const TrackArgs& a, int tile, unsigned char* dyn) {
     constexpr int NT = TW * TH;
     static_assert(!COMP || ANALYTIC, "compensated accumulation: analytic Jacobian");
     static_assert(TW % 8 == 0 && TH % 4 == 0 && NT % 32 == 0 && NT <= 256, "tile of 8 x 4 pixel warps");
     static_assert(TW != 16 || TH == 8 || TH == 16, "16-wide CTAs: 8-row bands");
-    static_assert(!TMA || (BATCH == kBatch && TW == kTW && TH == kTH),
-                  "the TMA staging gathers batches of kBatch records for 16 x 16 tiles");
-    static_assert(BATCH % 128 == 0 && BATCH <= 512, "batch of 128, 256 or 512 Gaussians");
-    static_assert(!ANALYTIC || (!TMA && !REF_LAYOUT), "analytic Jacobian: packed records, plain staging");
-    BodyBatch<TW, TH, BATCH, ANALYTIC>& sb = *reinterpret_cast<BodyBatch<TW, TH, BATCH, ANALYTIC>*>(dyn);
+    static_assert(!ANALYTIC || !REF_LAYOUT, "analytic Jacobian: packed records");
+    using Stage = BodyStage<TW, TH, ANALYTIC>;
+    Stage& ws = reinterpret_cast<Stage*>(dyn)[threadIdx.x >> 5];
     __shared__ float s_red[NT / 32][32];
     __shared__ float s_red_lo[COMP ? NT / 32 : 1][32];
-    __shared__ uint32_t s_nmax;
-    TmaStage& ts = body_tma_stage<TW, TH, BATCH, ANALYTIC>(dyn);
-    TmaState tm;
 
     // the list tile and this CTA's pixel block in it
     const int split = a.split > 1 ? a.split : 1;
@@ -702,8 +461,9 @@ __device__ __forceinline__ void track_tile_body(const TrackArgs& a, const RecMap
     const int tid = threadIdx.x;
     // each warp covers an 8 x 4 pixel block (compact footprint: less divergence)
     const int wq = tid >> 5, lq = tid & 31;
-    const int x = px0 + (wq % (TW / 8)) * 8 + (lq & 7), y = py0 + (wq / (TW / 8)) * 4 + (lq >> 3);
-    const float x0 = (float)px0, y0 = (float)py0;
+    const int wx0 = px0 + (wq % (TW / 8)) * 8, wy0 = py0 + (wq / (TW / 8)) * 4;
+    const int x = wx0 + (lq & 7), y = wy0 + (lq >> 3);
+    const float x0 = (float)wx0, y0 = (float)wy0;
     const bool in_bounds = (x < a.W && y < a.H);
     const size_t p = (size_t)y * a.W + x;
     uint2 range = a.ranges[lt];
@@ -744,194 +504,102 @@ __device__ __forceinline__ void track_tile_body(const TrackArgs& a, const RecMap
         for (int k = 0; k < 6; ++k) s_jd[k][tid] = 0.f;
     }
     if (n > 0) {
-        if (TMA) tma_begin(a, maps, ts, range.x, n, tm);
-        for (int base = 0; base < n; base += BATCH) {
-            if (__syncthreads_and(done)) break;
-            int cnt;
-            if constexpr (TMA)
-                cnt = stage_batch_tma<true>(a, maps, sb, ts, range.x, base, n, x0, y0, tm);
-            else
-                cnt = stage_batch<REF_LAYOUT, true, FUSED ? kStageDeriv : kStageNone, TW, TH>(a, sb, range.x,
-                                                                                                 base, n, x0, y0);
-            build_warp_bitmaps(sb, cnt);
-            if (FUSED && !done) {
-                int last_j = -1;
-                // one staged Gaussian with its conic-form gradient (dl0, dl1):
-                // returns false when the pixel terminates
-                auto blend_jac = [&](int j, float dx, float dy, float dl0, float dl1, float v) -> bool {
-                    const float4 rB = sb.B[j];
-                    const float raw = gauss_weight(rB.z, v);
-                    const float alpha = fminf(0.99f, raw);
-                    if (alpha < kInv255) return true;
-                    const float test_T = T * (1.0f - alpha);
-                    if (test_T < 0.0001f) return false;
-                    const float4 rC = sb.C[j];
-                    const float cB = sb.D[j];
-                    const float aT = alpha * T;
-                    if constexpr (COMP) {
-                        kahan_add(cr, ccr, rC.z * aT);
-                        kahan_add(cg, ccg, rC.w * aT);
-                        kahan_add(cb, ccb, cB * aT);
-                    } else {
-                        cr += rC.z * aT;
-                        cg += rC.w * aT;
-                        cb += cB * aT;
-                    }
-                    const float inv1m = rcp_approx(1.0f - alpha);
-                    const float kf = (raw > 0.99f) ? 0.0f : -0.5f * alpha;
-                    const float kfi = kf * inv1m;
-                    const float kT = kf * T;
-                    const float2 w0 = make_float2(kT * rC.z + kfi * cr, kT * rC.z + kfi * cr);
-                    const float2 w1 = make_float2(kT * rC.w + kfi * cg, kT * rC.w + kfi * cg);
-                    const float2 w2 = make_float2(kT * cB + kfi * cb, kT * cB + kfi * cb);
-                    const float2 wi = make_float2(kfi, kfi);
-                    const float cu = 2.0f * dl0, cv = 2.0f * dl1, ca = dx * dx, cb2 = 2.0f * dx * dy, cc = dy * dy;
-                    const float2 cu2 = make_float2(cu, cu), cv2 = make_float2(cv, cv), ca2 = make_float2(ca, ca),
-                                 cb22 = make_float2(cb2, cb2), cc2 = make_float2(cc, cc);
-#pragma unroll
-                    for (int m = 0; m < 3; ++m) {
-                        // dv/dpose = cu du + cv dv + ca da + cb2 db + cc dc for pose pair m
-                        const DerivPair d = deriv_pair(sb.X, j, m);
-                        float2 gv = __fmul2_rn(cu2, d.du);
-                        gv = __ffma2_rn(cv2, d.dv, gv);
-                        gv = __ffma2_rn(ca2, d.da, gv);
-                        gv = __ffma2_rn(cb22, d.db, gv);
-                        gv = __ffma2_rn(cc2, d.dc, gv);
-                        fs1[0][m] = __ffma2_rn(w0, gv, fs1[0][m]);
-                        fs1[1][m] = __ffma2_rn(w1, gv, fs1[1][m]);
-                        fs1[2][m] = __ffma2_rn(w2, gv, fs1[2][m]);
-                        fs2[m] = __ffma2_rn(wi, gv, fs2[m]);
-                    }
-                    if (T > 0.5f && test_T < 0.5f) {
-                        const float4 rA = sb.A[j];
-                        depth = depth_at(rB.w, rA.x, xf, rC.x, rA.y, yf, rC.y);
-                        // d depth = d z + phat . d(dx, dy) + (dx, dy) . d phat, with
-                        // d phat = (dp_x / z^2 - 2 x dp_z / z^3, dp_y / z^2 - 2 y dp_z / z^3)
-                        const float z = rB.w, x = sb.X[7][j].z, y = sb.X[7][j].w;
-                        const float iz = __frcp_rn(z), iz2 = iz * iz, iz3 = iz2 * iz;
-#pragma unroll
-                        for (int k = 0; k < 6; ++k) {
-                            const float dpx = k == 0 ? -1.f : (k == 4 ? -z : (k == 5 ? y : 0.f));
-                            const float dpy = k == 1 ? -1.f : (k == 3 ? z : (k == 5 ? -x : 0.f));
-                            const float dpz = k == 2 ? -1.f : (k == 3 ? -y : (k == 4 ? x : 0.f));
-                            const float dphx = dpx * iz2 - 2.f * x * iz3 * dpz;
-                            const float dphy = dpy * iz2 - 2.f * y * iz3 * dpz;
-                            const DerivPair d = deriv_pair(sb.X, j, k >> 1);
-                            const float du_k = (k & 1) ? d.du.y : d.du.x;
-                            const float dv_k = (k & 1) ? d.dv.y : d.dv.x;
-                            s_jd[k][tid] = dpz + rC.x * du_k + dx * dphx + rC.y * dv_k + dy * dphy;
-                        }
-                    }
-                    T = test_T;
-                    last_j = j;
-                    return true;
-                };
-                for (int g = 0; g * 32 < cnt && !done; ++g) {
-                    uint32_t bits = sb.bm[wq][g];
-                    while (bits) {
-                        const int j0 = g * 32 + __ffs(bits) - 1;
-                        bits &= bits - 1;
-                        if (bits) {
-                            const int j1 = g * 32 + __ffs(bits) - 1;
-                            bits &= bits - 1;
-                            const float4 rA0 = sb.A[j0], rA1 = sb.A[j1];
-                            const float2 rB0 = *reinterpret_cast<const float2*>(&sb.B[j0]);
-                            const float2 rB1 = *reinterpret_cast<const float2*>(&sb.B[j1]);
-                            const float dx0 = rA0.x - xf, dy0 = rA0.y - yf;
-                            const float dx1 = rA1.x - xf, dy1 = rA1.y - yf;
-                            float l00, l01, l10, l11;
-                            const float v0 = conic_form(rA0.z, rA0.w, rB0.x, dx0, dy0, l00, l01);
-                            const float v1 = conic_form(rA1.z, rA1.w, rB1.x, dx1, dy1, l10, l11);
-                            const bool k0 = !(v0 > rB0.y || v0 <= 0.0f);
-                            const bool k1 = !(v1 > rB1.y || v1 <= 0.0f);
-                            if (k0 && !blend_jac(j0, dx0, dy0, l00, l01, v0)) {
-                                done = true;
-                                break;
-                            }
-                            if (k1 && !blend_jac(j1, dx1, dy1, l10, l11, v1)) {
-                                done = true;
-                                break;
-                            }
-                        } else {
-                            const float4 rA = sb.A[j0];
-                            const float2 rB = *reinterpret_cast<const float2*>(&sb.B[j0]);
-                            const float dx = rA.x - xf, dy = rA.y - yf;
-                            float l0, l1;
-                            const float v = conic_form(rA.z, rA.w, rB.x, dx, dy, l0, l1);
-                            if (!(v > rB.y || v <= 0.0f) && !blend_jac(j0, dx, dy, l0, l1, v)) {
-                                done = true;
-                                break;
-                            }
-                        }
-                    }
+        int last_j = -1;  // staged slot of the last blended Gaussian of this round
+        auto round_end = [&]() {
+            if (last_j >= 0) last = (uint32_t)__float_as_int(ws.E[last_j].y) + 1u;
+            last_j = -1;
+        };
+        if constexpr (FUSED) {
+            // one staged Gaussian with its conic-form gradient (dl0, dl1)
+            auto blend_jac = [&](int j, const float4& rA, const float4& rB, float dx, float dy, float dl0, float dl1, float v,
+                                 float raw) {
+                const float alpha = fminf(0.99f, raw);
+                if (done || v > rB.y || v <= 0.0f || alpha < kInv255) return;
+                const float test_T = T * (1.0f - alpha);
+                if (test_T < 0.0001f) {
+                    done = true;
+                    return;
                 }
-                if (last_j >= 0) last = (uint32_t)sb.orig[last_j] + 1u;
-            }
-            if (!FUSED && !done) {
-                int last_j = -1;  // staged slot of the last blended Gaussian in this batch
-                // one staged Gaussian: returns false when the pixel terminates
-                auto blend = [&](int j, float dx, float dy, float v) -> bool {
-                    const float4 rB = sb.B[j];
-                    const float alpha = gauss_alpha(rB.z, v);
-                    if (alpha < kInv255) return true;
-                    const float test_T = T * (1.0f - alpha);
-                    if (test_T < 0.0001f) return false;
-                    const float4 rC = sb.C[j];
-                    const float aT = alpha * T;
+                const float4 rC = ws.C[j];
+                const float cB = ws.E[j].x;
+                const float aT = alpha * T;
+                if constexpr (COMP) {
+                    kahan_add(cr, ccr, rC.z * aT);
+                    kahan_add(cg, ccg, rC.w * aT);
+                    kahan_add(cb, ccb, cB * aT);
+                } else {
                     cr += rC.z * aT;
                     cg += rC.w * aT;
-                    cb += sb.D[j] * aT;
-                    if (T > 0.5f && test_T < 0.5f) depth = depth_at(rB.w, sb.A[j].x, xf, rC.x, sb.A[j].y, yf, rC.y);
-                    T = test_T;
-                    last_j = j;
-                    return true;
-                };
-                // the warp's own entries (its bitmap), two per iteration: both
-                // quadratic forms are evaluated before the (mostly rejecting)
-                // branches, in list order
-                for (int g = 0; g * 32 < cnt && !done; ++g) {
-                    uint32_t bits = sb.bm[wq][g];
-                    while (bits) {
-                        const int j0 = g * 32 + __ffs(bits) - 1;
-                        bits &= bits - 1;
-                        if (bits) {
-                            const int j1 = g * 32 + __ffs(bits) - 1;
-                            bits &= bits - 1;
-                            const float4 rA0 = sb.A[j0], rA1 = sb.A[j1];
-                            const float2 rB0 = *reinterpret_cast<const float2*>(&sb.B[j0]);
-                            const float2 rB1 = *reinterpret_cast<const float2*>(&sb.B[j1]);
-                            const float dx0 = rA0.x - xf, dy0 = rA0.y - yf;
-                            const float dx1 = rA1.x - xf, dy1 = rA1.y - yf;
-                            float q0, q1;
-                            const float v0 = conic_form(rA0.z, rA0.w, rB0.x, dx0, dy0, q0, q1);
-                            const float v1 = conic_form(rA1.z, rA1.w, rB1.x, dx1, dy1, q0, q1);
-                            const bool k0 = !(v0 > rB0.y || v0 <= 0.0f);
-                            const bool k1 = !(v1 > rB1.y || v1 <= 0.0f);
-                            if (k0 && !blend(j0, dx0, dy0, v0)) {
-                                done = true;
-                                break;
-                            }
-                            if (k1 && !blend(j1, dx1, dy1, v1)) {
-                                done = true;
-                                break;
-                            }
-                        } else {
-                            const float4 rA = sb.A[j0];
-                            const float2 rB = *reinterpret_cast<const float2*>(&sb.B[j0]);
-                            const float dx = rA.x - xf, dy = rA.y - yf;
-                            float q0, q1;
-                            const float v = conic_form(rA.z, rA.w, rB.x, dx, dy, q0, q1);
-                            if (!(v > rB.y || v <= 0.0f) && !blend(j0, dx, dy, v)) {
-                                done = true;
-                                break;
-                            }
-                        }
+                    cb += cB * aT;
+                }
+                const float inv1m = rcp_approx(1.0f - alpha);
+                const float kf = (raw > 0.99f) ? 0.0f : -0.5f * alpha;
+                const float kfi = kf * inv1m;
+                const float kT = kf * T;
+                const float2 w0 = make_float2(kT * rC.z + kfi * cr, kT * rC.z + kfi * cr);
+                const float2 w1 = make_float2(kT * rC.w + kfi * cg, kT * rC.w + kfi * cg);
+                const float2 w2 = make_float2(kT * cB + kfi * cb, kT * cB + kfi * cb);
+                const float2 wi = make_float2(kfi, kfi);
+                const float cu = 2.0f * dl0, cv = 2.0f * dl1, ca = dx * dx, cb2 = 2.0f * dx * dy, cc = dy * dy;
+                const float2 cu2 = make_float2(cu, cu), cv2 = make_float2(cv, cv), ca2 = make_float2(ca, ca),
+                             cb22 = make_float2(cb2, cb2), cc2 = make_float2(cc, cc);
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    // dv/dpose = cu du + cv dv + ca da + cb2 db + cc dc for pose pair m
+                    const DerivPair d = deriv_pair(ws.X[j], m);
+                    float2 gv = __fmul2_rn(cu2, d.du);
+                    gv = __ffma2_rn(cv2, d.dv, gv);
+                    gv = __ffma2_rn(ca2, d.da, gv);
+                    gv = __ffma2_rn(cb22, d.db, gv);
+                    gv = __ffma2_rn(cc2, d.dc, gv);
+                    fs1[0][m] = __ffma2_rn(w0, gv, fs1[0][m]);
+                    fs1[1][m] = __ffma2_rn(w1, gv, fs1[1][m]);
+                    fs1[2][m] = __ffma2_rn(w2, gv, fs1[2][m]);
+                    fs2[m] = __ffma2_rn(wi, gv, fs2[m]);
+                }
+                if (T > 0.5f && test_T < 0.5f) {
+                    depth = depth_at(rB.w, rA.x, xf, rC.x, rA.y, yf, rC.y);
+                    // d depth = d z + phat . d(dx, dy) + (dx, dy) . d phat, with
+                    // d phat = (dp_x / z^2 - 2 x dp_z / z^3, dp_y / z^2 - 2 y dp_z / z^3)
+                    const float z = rB.w, x = ws.X[j][7].z, y = ws.X[j][7].w;
+                    const float iz = __frcp_rn(z), iz2 = iz * iz, iz3 = iz2 * iz;
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) {
+                        const float dpx = k == 0 ? -1.f : (k == 4 ? -z : (k == 5 ? y : 0.f));
+                        const float dpy = k == 1 ? -1.f : (k == 3 ? z : (k == 5 ? -x : 0.f));
+                        const float dpz = k == 2 ? -1.f : (k == 3 ? -y : (k == 4 ? x : 0.f));
+                        const float dphx = dpx * iz2 - 2.f * x * iz3 * dpz;
+                        const float dphy = dpy * iz2 - 2.f * y * iz3 * dpz;
+                        const DerivPair d = deriv_pair(ws.X[j], k >> 1);
+                        const float du_k = (k & 1) ? d.du.y : d.du.x;
+                        const float dv_k = (k & 1) ? d.dv.y : d.dv.x;
+                        s_jd[k][tid] = dpz + rC.x * du_k + dx * dphx + rC.y * dv_k + dy * dphy;
                     }
                 }
-                if (last_j >= 0) last = (uint32_t)sb.orig[last_j] + 1u;
-            }
+                T = test_T;
+                last_j = j;
+            };
+            walk_list<REF_LAYOUT, kMasksNone, kStageDeriv>(a, ws, range.x, n, x0, y0, xf, yf, done, blend_jac, round_end);
+        } else {
+            auto blend = [&](int j, const float4& rA, const float4& rB, float dx, float dy, float, float, float v, float raw) {
+                const float alpha = fminf(0.99f, raw);
+                if (done || v > rB.y || v <= 0.0f || alpha < kInv255) return;
+                const float test_T = T * (1.0f - alpha);
+                if (test_T < 0.0001f) {
+                    done = true;
+                    return;
+                }
+                const float4 rC = ws.C[j];
+                const float aT = alpha * T;
+                cr += rC.z * aT;
+                cg += rC.w * aT;
+                cb += ws.E[j].x * aT;
+                if (T > 0.5f && test_T < 0.5f) depth = depth_at(rB.w, rA.x, xf, rC.x, rA.y, yf, rC.y);
+                T = test_T;
+                last_j = j;
+            };
+            walk_list<REF_LAYOUT, RENDER_ONLY ? kMasksNone : kMasksKeep, kStageNone>(a, ws, range.x, n, x0, y0, xf, yf, done, blend, round_end);
         }
-        if (TMA) tma_drain(a, ts, tm);
         if (inside) {
             final_T = T;
             n_contrib = last;
@@ -1021,14 +689,6 @@ __device__ __forceinline__ void track_tile_body(const TrackArgs& a, const RecMap
     }
 
     // ------------------- pass 2 (reference Jacobian): per-Gaussian terms ---
-    int nmax = 0;
-    if constexpr (!FUSED) {
-        if (tid == 0) s_nmax = 0;
-        __syncthreads();
-        if (do_jac && n_contrib > 0) atomicMax(&s_nmax, n_contrib);
-        __syncthreads();
-        nmax = (int)min((uint32_t)n, s_nmax);
-    }
     if constexpr (ANALYTIC) {
         // Colour Jacobian jc (3 x 6) of the pixel from the fused pass's sums:
         // jc = S1 - C S2 (C: the final colour with background); jd: the depth
@@ -1066,99 +726,80 @@ __device__ __forceinline__ void track_tile_body(const TrackArgs& a, const RecMap
             }
         }
     } else {
-            // rem = final colour minus the colour accumulated so far (running)
-            float prod_alpha = 1.f, remr = cr, remg = cg, remb = cb;
-            bool depth_pending = img_depth > 0.5f;  // the depth term is added once, where T first falls to 0.5
-            bool done2 = !do_jac;
-            if (TMA) tma_begin(a, maps, ts, range.x, nmax, tm);
-            for (int base = 0; base < nmax; base += BATCH) {
-                if (__syncthreads_and(done2)) break;
-                int cnt;
-                if constexpr (TMA)
-                    cnt = stage_batch_tma<false>(a, maps, sb, ts, range.x, base, nmax, x0, y0, tm);
-                else
-                    cnt = stage_batch<REF_LAYOUT, false, kStageRay, TW, TH>(a, sb, range.x, base, nmax, x0, y0);
-                build_warp_bitmaps(sb, cnt);
-                if (!done2) {
-                    for (int g = 0; g * 32 < cnt && !done2; ++g) {
-                        for (uint32_t bits = sb.bm[wq][g]; bits; bits &= bits - 1) {
-                            const int j = g * 32 + __ffs(bits) - 1;
-                        if (sb.orig[j] >= (int)n_contrib) {
-                            done2 = true;
-                            break;
-                        }
-                        const float4 rA = sb.A[j];
-                        const float4 rB = sb.B[j];
-                        const float dx = rA.x - xf, dy = rA.y - yf;
-                        float dl0, dl1;
-                        const float v = conic_form(rA.z, rA.w, rB.x, dx, dy, dl0, dl1);
-                        if (v > rB.y) continue;
-                        const float alpha = gauss_alpha(rB.z, v);
-                        if (alpha < kInv255) continue;
-                        const float4 rC = sb.C[j];
-                        const float4 rE = sb.X[0][j];
-                        const float d = depth_fast(rB.w, dx, rC.x, dy, rC.y, rA.x, xf, rA.y, yf);
-                        float da0 = rC.z * prod_alpha, da1 = rC.w * prod_alpha, da2 = sb.D[j] * prod_alpha;
-                        remr -= alpha * da0;
-                        remg -= alpha * da1;
-                        remb -= alpha * da2;
-                        const float inv1m = rcp_approx(1.0f - alpha);
-                        da0 -= remr * inv1m;
-                        da1 -= remg * inv1m;
-                        da2 -= remb * inv1m;
-                        // The reference's per-Gaussian row is u = (jt, d (r x jt)) with
-                        // jt = g / d, g = (fx dl0, fy dl1, -fx rgx dl0 - fy rgy dl1) and
-                        // r = (rgx, rgy, 1): the same vector as (g / d, r x g).
-                        const float g0 = fx * dl0, g1 = fy * dl1, g2 = rE.z * dl0 + rE.w * dl1;
-                        const float inv_d = rcp_approx(d);
-                        const float u0 = g0 * inv_d, u1 = g1 * inv_d, u2 = g2 * inv_d;
-                        const float u3 = rE.y * g2 - g1, u4 = g0 - rE.x * g2, u5 = rE.x * g1 - rE.y * g0;
-                        const float w = wc * alpha * alpha * (da0 * da0 + da1 * da1 + da2 * da2);
-                        {
-                            const float u[6] = {u0, u1, u2, u3, u4, u5};
-                            int idx = 0;
-        #pragma unroll
-                            for (int i = 0; i < 6; ++i) {
-                                const float wu = w * u[i];
-        #pragma unroll
-                                for (int k = i; k < 6; ++k) A[idx++] += wu * u[k];
-                            }
-                        }
-                        const float coef = -wc * alpha * (da0 * e0 + da1 * e1 + da2 * e2);
-                        bv[0] += coef * u0;
-                        bv[1] += coef * u1;
-                        bv[2] += coef * u2;
-                        bv[3] += coef * u3;
-                        bv[4] += coef * u4;
-                        bv[5] += coef * u5;
-                        prod_alpha *= (1.0f - alpha);
-                        if (depth_pending && prod_alpha <= 0.5f) {
-                            // the depth term wd * derr * r: its rotation part d (r x r) is zero
-                            depth_pending = false;
-                            const float r[3] = {rE.x, rE.y, 1.0f};
-                            int idx = 0;
-        #pragma unroll
-                            for (int i = 0; i < 3; ++i) {
-        #pragma unroll
-                                for (int jj = i; jj < 6; ++jj) {
-                                    if (jj < 3) A[idx] += wd * r[i] * r[jj];
-                                    ++idx;
-                                }
-                            }
-                            bv[0] += wd * derr * rE.x;
-                            bv[1] += wd * derr * rE.y;
-                            bv[2] += wd * derr;
-                        }
-                        if (prod_alpha < 0.001f) {
-                            done2 = true;
-                            break;
-                        }
-                    }
+        // rem = final colour minus the colour accumulated so far (running)
+        float prod_alpha = 1.f, remr = cr, remg = cg, remb = cb;
+        bool depth_pending = img_depth > 0.5f;  // the depth term is added once, where T first falls to 0.5
+        bool done2 = !do_jac || n_contrib == 0;
+        // the entries past the last contributor of the warp's pixels are not needed
+        const int nmax = (int)min((uint32_t)n, __reduce_max_sync(kFullMask, do_jac ? n_contrib : 0u));
+        auto rank_one = [&](int j, const float4& rA, const float4& rB, float dx, float dy, float dl0, float dl1, float v,
+                            float raw) {
+            if (done2) return;
+            if (rB.y != -INFINITY && __float_as_int(ws.E[j].y) >= (int)n_contrib) {
+                done2 = true;
+                return;
+            }
+            const float alpha = fminf(0.99f, raw);
+            if (v > rB.y || alpha < kInv255) return;
+            const float4 rC = ws.C[j];
+            const float4 rE = ws.X[j][0];
+            const float d = depth_fast(rB.w, dx, rC.x, dy, rC.y, rA.x, xf, rA.y, yf);
+            float da0 = rC.z * prod_alpha, da1 = rC.w * prod_alpha, da2 = ws.E[j].x * prod_alpha;
+            remr -= alpha * da0;
+            remg -= alpha * da1;
+            remb -= alpha * da2;
+            const float inv1m = rcp_approx(1.0f - alpha);
+            da0 -= remr * inv1m;
+            da1 -= remg * inv1m;
+            da2 -= remb * inv1m;
+            // The reference's per-Gaussian row is u = (jt, d (r x jt)) with
+            // jt = g / d, g = (fx dl0, fy dl1, -fx rgx dl0 - fy rgy dl1) and
+            // r = (rgx, rgy, 1): the same vector as (g / d, r x g).
+            const float g0 = fx * dl0, g1 = fy * dl1, g2 = rE.z * dl0 + rE.w * dl1;
+            const float inv_d = rcp_approx(d);
+            const float u0 = g0 * inv_d, u1 = g1 * inv_d, u2 = g2 * inv_d;
+            const float u3 = rE.y * g2 - g1, u4 = g0 - rE.x * g2, u5 = rE.x * g1 - rE.y * g0;
+            const float w = wc * alpha * alpha * (da0 * da0 + da1 * da1 + da2 * da2);
+            {
+                const float u[6] = {u0, u1, u2, u3, u4, u5};
+                int idx = 0;
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+                    const float wu = w * u[i];
+#pragma unroll
+                    for (int k = i; k < 6; ++k) A[idx++] += wu * u[k];
                 }
             }
-        }
+            const float coef = -wc * alpha * (da0 * e0 + da1 * e1 + da2 * e2);
+            bv[0] += coef * u0;
+            bv[1] += coef * u1;
+            bv[2] += coef * u2;
+            bv[3] += coef * u3;
+            bv[4] += coef * u4;
+            bv[5] += coef * u5;
+            prod_alpha *= (1.0f - alpha);
+            if (depth_pending && prod_alpha <= 0.5f) {
+                // the depth term wd * derr * r: its rotation part d (r x r) is zero
+                depth_pending = false;
+                const float r[3] = {rE.x, rE.y, 1.0f};
+                int idx = 0;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+#pragma unroll
+                    for (int jj = i; jj < 6; ++jj) {
+                        if (jj < 3) A[idx] += wd * r[i] * r[jj];
+                        ++idx;
+                    }
+                }
+                bv[0] += wd * derr * rE.x;
+                bv[1] += wd * derr * rE.y;
+                bv[2] += wd * derr;
+            }
+            if (prod_alpha < 0.001f) done2 = true;
+        };
+        if (nmax > 0)
+            walk_list<REF_LAYOUT, kMasksUse, kStageRay>(a, ws, range.x, nmax, x0, y0, xf, yf, done2, rank_one, [] {});
     }
-    if (TMA) tma_drain(a, ts, tm);
 
     // --------------------------- tile reduction ------------------------------
     float vals[32];

@@ -104,21 +104,16 @@ int fvgs_session_set_precision(fvgs_session* s, int precision);
 /*
  * Launch autotuner of the Jacobian kernel (batching form).  The kernel has
  * eight launch variants with the same arithmetic in the same order:
- *   0: four CTAs of 256 threads per SM at 64 registers, batches of 256
- *      Gaussians staged in shared memory;
- *   1: three CTAs per SM at 80 registers;
- *   2: as 0, each batch of records gathered into shared memory by TMA while
- *      the previous batch is blended;
- *   3, 4: as 0 with batches of 128 and 512 Gaussians;
- *   5, 6: each 16 x 16 tile's list run by 2 CTAs of 16 x 8 pixels (5) or 4
- *      CTAs of 8 x 8 pixels (6), batches of 128 Gaussians: more CTAs for the
- *      few hundred tiles of a coarse pyramid level (16 x 16 tiles without
- *      compensated sums only; otherwise they run as 3);
- *   7: two CTAs per SM at 128 registers.
- * With the analytic Jacobian (whose single fused pass holds the colour
- * Jacobian's sums) every variant runs one CTA per SM fewer: 0, 3, 4 at three
- * CTAs and 80 registers, 1 at two CTAs and 128 registers, 7 at two CTAs with
- * batches of 128; 2 runs as 0.
+ *   0, 3, 6: each 16 x 16 tile run by 4 CTAs of 8 x 8 pixels (two warps), at
+ *      the largest, middle and smallest register budget;
+ *   2, 4, 5: the same by 2 CTAs of 16 x 8 pixels;
+ *   1, 7: one CTA per tile, at the largest and smallest budget.
+ * The budgets are 128, 96 and 80 registers per thread with the analytic
+ * Jacobian (whose fused pass holds the colour Jacobian's sums) and 96, 80 and
+ * 64 with the reference's.  Every warp walks its tile's list on its own, so
+ * the forms differ in how tiles fill the SMs and in spilled registers only.
+ * Compensated sums (precision form) and tiles of 8 x 8 and 32 x 8 pixels have
+ * one form each.
  * Which is faster depends on the map and frame.  On the first frame of a new
  * frame shape of a pyramid level (fvgs_track_frame, fvgs_frame_submit) the
  * session bins the frame at the request's pose, times every variant on that
@@ -306,13 +301,15 @@ int fvgs_session_set_track_tiles(fvgs_session* s, int level, int tile_w, int til
  * sessions' binning state allows.  poses[i] is read and overwritten.  A
  * session whose instance buffers overflow is repeated alone on the plain
  * path after they grow.
- * Each level's tile shape and staging batch (128, 256 or 512 Gaussians per
- * shared-memory batch) belong to the batch and are pushed to its sessions
- * (fvgs_session_set_track_tiles and the launch variant), so a session's plain
- * frames give the batched result bit for bit.  fvgs_batch_set_level sets
- * them; fvgs_batch_autotune times the persistent launch for every shape x
+ * Each level's tile shape belongs to the batch and is pushed to its sessions
+ * (fvgs_session_set_track_tiles), so a session's plain frames give the
+ * batched result bit for bit.  The staging batch (128, 256 or 512 Gaussians)
+ * is accepted and reported, and changes neither results nor the launch: every
+ * warp stages 32 list entries at a time.  fvgs_batch_set_level sets both;
+ * fvgs_batch_autotune times the persistent launch for every shape x
  * batch (9 combinations) on every level the schedule uses, at the given
- * poses (reps launches each), and keeps the fastest per level; config_out
+ * poses (reps launches each), and keeps the fastest per level (another shape
+ * than 16 x 16 only when it is a quarter faster); config_out
  * (nullable, 3 ints per level: tile_w, tile_h, batch) and ms_out (nullable,
  * 9 floats per level: shapes 16x16, 8x8, 32x8, each with batches 128, 256,
  * 512) report the outcome.  fvgs_batch_stats: frames replayed / enqueued

@@ -324,3 +324,40 @@ def test_track_tiles_room_1m_hd(oracle, fvgs_lib, quirks):
               (e_sum_jtj, e_sum_jtr, np.mean(per <= 1e-4), per.size))
         assert e_sum_jtj <= JAC_RTOL and e_sum_jtr <= JAC_RTOL, (name, e_sum_jtj, e_sum_jtr)
         assert per.size > 150 and np.mean(per <= 1e-4) > 0.97, (name, np.sort(per)[-5:])
+
+
+@pytest.mark.parametrize("quirks", [REF, INTENDED], ids=["ref", "analytic"])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 65])
+@pytest.mark.parametrize("size", [(16, 16), (21, 13), (9, 5)])
+def test_track_jacobian_list_and_block_edges(oracle, fvgs_lib, n, size, quirks):
+    """Lists around a warp's staging round of 32 entries and frames whose 8 x 4
+    pixel blocks are partly or wholly outside the image; every launch form
+    gives the same bits."""
+    W, H = size
+    K = (30.0, 30.0, (W - 1) / 2.0, (H - 1) / 2.0)
+    rng = np.random.default_rng(1000 * n + W)
+    scene = S.cam_box(n, seed=n)
+    scene.positions[:, :2] = rng.uniform(-0.1, 0.1, (n, 2)) * scene.positions[:, 2:]
+    scene.scales[:] = rng.uniform(0.2, 0.6, (n, 3))
+    P = oracle.default_params(quirks)
+    pose = (np.zeros(3, np.float32), S.IDENTITY_Q)
+    start = S.perturb(pose, 0.3, 0.5, rng)
+    frame = make_frame(oracle, scene, pose, K, W, H, P)
+    b = oracle.prepare(scene, start, K, W, H, P)
+    r = oracle.track(b, frame, start, K, W, H, P, images=False)
+    with fvgs_lib.Session(n, W, H, fvgs_lib.default_params(quirks)) as s:
+        s.upload(scene)
+        s.set_frame(0, *frame)
+        out = []
+        for v in range(fvgs_lib.TRACK_VARIANTS):
+            s.set_track_variant(0, v)
+            out.append(s.track_jacobian(start, K, 0))
+    JtJ, Jtr = out[0]
+    for o in out[1:]:
+        np.testing.assert_array_equal(o[0], JtJ)
+        np.testing.assert_array_equal(o[1], Jtr)
+    if np.linalg.norm(r.JtJ) == 0.0:
+        assert not JtJ.any() and not Jtr.any()
+        return
+    assert rel_err(JtJ, r.JtJ) <= JAC_RTOL
+    assert rel_err(Jtr, r.Jtr) <= JAC_RTOL
