@@ -118,6 +118,7 @@ struct BinCtx {
     uint32_t* vals_home = nullptr;
     bool hist_ok = false;
     int hist_ntx = 0, hist_nty = 0, hist_tw = 0, hist_th = 0;
+    uint32_t n_hint = 0;  // instances of the grid's last binning whose status the host has read (0: none)
 };
 
 // Host-side binning state of every context and the active one (graph entry
@@ -434,6 +435,7 @@ void ctx_select(fvgs_session* s, int W, int H, int tw, int th) {
         c.tw = tw;
         c.th = th;
         c.hist_ok = false;
+        c.n_hint = 0;
     }
     s->bctx[pick].last_use = ++s->bctx_clock;
     ctx_load(s, pick);
@@ -510,6 +512,7 @@ int alloc_instances(fvgs_session* s, uint64_t cap) {
         }
         dev_free(s, s->sort.keys_alt, s->cap_inst);
         dev_free(s, s->sort.lookback, sort_lookback_words(s->cap_inst));
+        dev_free(s, s->seg.large_list, segsort_list_items(s->cap_inst, s->cap_tiles));
     }
     s->cap_inst = cap;
     FV_TRY(dev_alloc(s, &s->keys, cap));
@@ -524,6 +527,7 @@ int alloc_instances(fvgs_session* s, uint64_t cap) {
     FV_TRY(dev_alloc(s, &s->sort.keys_alt, cap));
     FV_TRY(dev_alloc(s, &s->sort.lookback, sort_lookback_words(cap)));
     FV_CK(cudaMemsetAsync(s->sort.lookback, 0, sizeof(uint64_t) * sort_lookback_words(cap), s->stream));
+    FV_TRY(dev_alloc(s, &s->seg.large_list, segsort_list_items(cap, s->cap_tiles)));
     s->sort.max_items = cap;
     s->sort.epoch = 1;
     return FVGS_OK;
@@ -729,8 +733,8 @@ int enqueue_bin(fvgs_session* s, const fvgs_intrinsics* K, int W, int H, int tw,
         inc.capacity = s->cap_inst;
         {
             KScope k(s, FVGS_K_SORT, 2);
-            FV_CK(launch_segsort(s->sort.keys_alt, s->keys, s->ranges, T, s->vals, s->seg, s->st, s->num_sms, inc,
-                                 s->stream));
+            FV_CK(launch_segsort(s->sort.keys_alt, s->keys, s->ranges, T, s->vals, s->seg, s->st,
+                                 s->bctx[s->bctx_cur].n_hint, s->num_sms, inc, s->stream));
         }
         s->keys_valid = false;
         if (P.quirks & FVGS_Q_RANGE_LAUNCH) {
@@ -860,6 +864,7 @@ int reset_status(fvgs_session* s) {
 int check_status(fvgs_session* s, int* retry) {
     *retry = 0;
     const DevStatus st = *s->h_st;
+    s->bctx[s->bctx_cur].n_hint = st.n_instances;
     if (st.flags & kErrTimeout) return FVGS_E_TIMEOUT;
     if (st.flags & kErrBounds) {
         // an incremental binning did not find the instance count of a tile:
@@ -1058,6 +1063,7 @@ int fvgs_session_create(const fvgs_params* params, int device, uint32_t capacity
     }
     FV_CK(cudaSetDevice(device));
     FV_CK(track_configure_device());
+    FV_CK(segsort_configure_device());
     fvgs_session* s = new (std::nothrow) fvgs_session();
     if (!s) return FVGS_E_NOMEM;
     s->params = P;
@@ -1116,7 +1122,6 @@ int fvgs_session_create(const fvgs_params* params, int device, uint32_t capacity
     s->enter_cap = std::max<uint32_t>(1u << 16, capacity_gaussians);
     FV_A(s->enter_keys, (size_t)s->enter_cap);
     FV_A(s->changed, (size_t)s->enter_cap);
-    FV_A(s->seg.large_list, (size_t)s->cap_tiles);
     FV_A(s->seg.large_ctrl, 4);  // [0..1] large-bucket list control, [2] scatter chunk counter
     // partial rows: four per tile (16 x 16 tiles run as 8 x 8 quarters), for
     // as many tiles as a frame may have

@@ -150,12 +150,15 @@ cudaError_t launch_tile_offsets(int* scratch, int ntx, int nty, bool hist, uint3
 cudaError_t launch_emit_scatter(const EmitArgs& a, uint32_t* fill, uint32_t* chunk_counter, int grid,
                                 const DevStatus* st, cudaStream_t s);
 // Per-tile sort of the composite keys (segsort.cu): writes the sorted Gaussian
-// indices to vals.  Tiles above 4096 instances go through a global merge sort
-// that uses tmp (capacity u64) as scratch.
+// indices to vals.  Tiles above 2^20 instances go through a global merge sort
+// that uses tmp (capacity u64) as scratch.  n_hint: the instances of the
+// grid's last binning as far as the host knows them (0: unknown); it chooses
+// the launch shape only.
 struct SegSortWork {
-    uint32_t* large_list;  // [T] tiles too large for one CTA
+    uint2* large_list;     // [segsort_list_items] key ranges (tile, range) of the tiles too large for one CTA
     uint32_t* large_ctrl;  // [2]: count, next
 };
+size_t segsort_list_items(uint64_t max_instances, int num_tiles);
 // Incremental mode inputs: the previous binning's ranges and sorted indices,
 // the entering instances per tile, and the current binning records.
 struct SegSortIncr {
@@ -169,8 +172,11 @@ struct SegSortIncr {
     uint64_t capacity;   // instance buffer size: previous ranges are clamped to it
 };
 cudaError_t launch_segsort(uint64_t* comp, uint64_t* tmp, const uint2* ranges, int num_tiles, uint32_t* vals,
-                           SegSortWork w, const DevStatus* st, int large_grid, const SegSortIncr& inc,
+                           SegSortWork w, const DevStatus* st, uint32_t n_hint, int num_sms, const SegSortIncr& inc,
                            cudaStream_t s);
+// Dynamic shared-memory limits of the per-tile sort on the current device;
+// once per device, before any launch or capture.
+cudaError_t segsort_configure_device();
 // Reference-format keys (tile << 32 | depth bits) of a tile-bucket binning,
 // rebuilt from its ranges, sorted indices and binning records with the
 // emission's arithmetic (the tracking path itself never reads them).

@@ -121,3 +121,33 @@ def test_binning_capacity_growth(oracle, fvgs_lib):
                     rng.uniform(0, 1, (n, 3)).astype(np.float32), np.full(n, 0.5, np.float32))
     b = _check(oracle, fvgs_lib, scene, (np.zeros(3), S.IDENTITY_Q), K, W, H, 0x4 | 0x8)
     assert b.keys.shape[0] > (1 << 20)
+
+
+@pytest.mark.parametrize("equal", [False, True], ids=["spread", "equal_depths"])
+@pytest.mark.parametrize("n", [1, 126, 127, 128, 512, 1536, 1537, 3072, 3073, 4096, 4097, 8192, 8193, 16384, 16385,
+                               40000, (1 << 20) + 5])
+def test_one_tile_sort_sizes(oracle, fvgs_lib, n, equal):
+    """One tile's list around the capacities of the per-tile sort's forms, full
+    and incremental (members leaving and entering between poses), and keys
+    that tie in depth and fall back to the index."""
+    W, H, K = 16, 16, (40.0, 40.0, 7.5, 7.5)
+    rng = np.random.default_rng(n)
+    scene = S.cam_box(n, seed=n)
+    z = scene.positions[:, 2]
+    scene.positions[:, :2] = rng.uniform(-0.21, 0.21, (n, 2)) * z[:, None]
+    if equal:
+        scene.positions[:] = [0.01, -0.02, 2.0]
+    P = oracle.default_params()
+    poses = [(np.zeros(3, np.float32), S.IDENTITY_Q)]
+    for deg, cm in ((0.05, 0.1), (1.0, 2.0), (0.0, 0.0)):
+        poses.append(S.perturb(poses[-1], deg, cm, rng))
+    with fvgs_lib.Session(n, W, H) as s:
+        s.upload(scene)
+        for pose in poses:
+            n_inst = s.project_bin(pose, K, W, H)
+            b = oracle.prepare(scene, pose, K, W, H, P)
+            keys, vals, ranges = s.download_binning(W, H)
+            assert n_inst == b.keys.shape[0]
+            np.testing.assert_array_equal(ranges, b.ranges)
+            np.testing.assert_array_equal(vals, b.vals)
+            np.testing.assert_array_equal(keys, b.keys)
