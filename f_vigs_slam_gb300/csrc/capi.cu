@@ -221,11 +221,6 @@ struct fvgs_session {
     size_t map_px = 0;
     float *m_final_T = nullptr, *m_color = nullptr, *m_depth = nullptr, *m_color_err = nullptr;
     uint32_t* m_n_contrib = nullptr;
-    uint32_t* m_max_contrib = nullptr;
-    uint32_t* m_bucket_base = nullptr;
-    uint32_t* m_bucket_total = nullptr;
-    float4* m_sampled = nullptr;
-    size_t m_sampled_slots = 0;
     int m_W = 0, m_H = 0;
 
     // map maintenance: second set of Gaussian planes (compaction target,
@@ -885,7 +880,7 @@ int check_status(fvgs_session* s, int* retry) {
 
 bool valid_pose(const fvgs_pose* p) { return p != nullptr; }
 
-int ensure_map_buffers(fvgs_session* s, size_t px, bool cap) {
+int ensure_map_buffers(fvgs_session* s, size_t px) {
     if (px > s->map_px) {
         dev_free(s, s->m_final_T, s->map_px);
         dev_free(s, s->m_n_contrib, s->map_px);
@@ -898,15 +893,6 @@ int ensure_map_buffers(fvgs_session* s, size_t px, bool cap) {
         FV_TRY(dev_alloc(s, &s->m_depth, px));
         FV_TRY(dev_alloc(s, &s->m_color_err, 3 * px));
         s->map_px = px;
-    }
-    // checkpoint slots: 8 per tile with MAP_CAP256, else one per 32 instances
-    // of every tile (bounded by capacity/32 + tiles)
-    const size_t slots = cap ? (size_t)s->cap_tiles16 * map_cap_buckets()
-                             : (size_t)(s->cap_inst / 32 + 1) + (size_t)s->cap_tiles16;
-    if (slots > s->m_sampled_slots) {
-        dev_free(s, s->m_sampled, s->m_sampled_slots * 256);
-        FV_TRY(dev_alloc(s, &s->m_sampled, slots * 256));
-        s->m_sampled_slots = slots;
     }
     return FVGS_OK;
 }
@@ -932,25 +918,18 @@ int enqueue_map(fvgs_session* s, const fvgs_intrinsics* K, const FrameLevel& f, 
     ma.bg[0] = P.bg[0];
     ma.bg[1] = P.bg[1];
     ma.bg[2] = P.bg[2];
-    ma.bucket_base = cap ? nullptr : s->m_bucket_base;
-    ma.sampled = s->m_sampled;
     ma.final_T = s->m_final_T;
     ma.n_contrib = s->m_n_contrib;
     ma.color = s->m_color;
     ma.depth = s->m_depth;
     ma.color_err = s->m_color_err;
-    ma.max_contrib = s->m_max_contrib;
     ma.delta2d = s->delta2d;
     ma.w_depth = P.w_depth;
     ma.w_dist = P.w_dist;
-    if (!cap) {
-        KScope k(s, FVGS_K_SCAN, 1);
-        FV_CK(launch_bucket_scan(s->ranges, ntx * nty, s->m_bucket_base, s->m_bucket_total, s->stream));
-    }
     FV_CK(cudaMemsetAsync(s->delta2d, 0, sizeof(float) * 16 * (size_t)s->n_g, s->stream));
     {
         KScope k(s, FVGS_K_MAP_FWD, 1);
-        FV_CK(launch_map_forward(ma, cap, s->stream));
+        FV_CK(launch_map_forward(ma, s->stream));
     }
     {
         KScope k(s, FVGS_K_MAP_BWD, 1);
@@ -965,6 +944,7 @@ int enqueue_map(fvgs_session* s, const fvgs_intrinsics* K, const FrameLevel& f, 
     ua.cap = s->cap_g;
     ua.n = (int)s->n_g;
     ua.delta2d = s->delta2d;
+    ua.counts = s->counts;
     ua.pose = s->pose;
     ua.K = *K;
     ua.lambda_iso = P.lambda_iso;
@@ -981,7 +961,7 @@ int enqueue_map(fvgs_session* s, const fvgs_intrinsics* K, const FrameLevel& f, 
     }
     {
         KScope k(s, FVGS_K_MAP_UPDATE, 1);
-        FV_CK(launch_map_update(ua, s->st, s->stream));
+        FV_CK(launch_map_update(ua, s->st, s->num_sms, s->stream));
     }
     s->m_W = f.W;
     s->m_H = f.H;
@@ -1134,9 +1114,6 @@ int fvgs_session_create(const fvgs_params* params, int device, uint32_t capacity
     FV_A(s->sort.ctrl, sort_ctrl_words());
     FV_A(s->adam, 9 * N);
     FV_A(s->delta2d, 16 * N);
-    FV_A(s->m_max_contrib, (size_t)s->cap_tiles);
-    FV_A(s->m_bucket_base, (size_t)s->cap_tiles);
-    FV_A(s->m_bucket_total, 1);
     FV_A(s->pos_alt, N);
     FV_A(s->scale_alt, N);
     FV_A(s->rot_alt, N);
@@ -1946,7 +1923,7 @@ int prepare_request(fvgs_session* s, const Request& r) {
     }
     if (r.eta >= 0.f) {
         const FrameLevel& f = s->lv[r.map_level];
-        FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H, (s->params.quirks & FVGS_Q_MAP_CAP256) != 0));
+        FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H));
     }
     for (int l = kMaxLevels - 1; l >= 0; --l)
         if (r.iters[l] > 0 && needs_tuning(s, l)) FV_TRY(autotune_track(s, &r.pose, &r.K[l], l, 5));
@@ -2052,7 +2029,7 @@ int fvgs_frame_wait(fvgs_session* s, fvgs_pose* pose, double* last_step) {
     for (int attempt = 0; retry && attempt < 4; ++attempt) {
         if (s->req.eta >= 0.f) {
             const FrameLevel& f = s->lv[s->req.map_level];
-            FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H, (s->params.quirks & FVGS_Q_MAP_CAP256) != 0));
+            FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H));
         }
         *s->h_pose = s->req.pose;
         ++s->frames_eager;
@@ -2822,7 +2799,7 @@ int fvgs_map_step(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics*
     if (!f.rgb) return FVGS_E_STATE;
     FV_CK(cudaSetDevice(s->device));
     const bool cap = (s->params.quirks & FVGS_Q_MAP_CAP256) != 0;
-    FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H, cap));
+    FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H));
     for (int attempt = 0; attempt < 4; ++attempt) {
         FV_TRY(reset_status(s));
         FV_TRY(set_pose(s, pose));
@@ -2835,7 +2812,7 @@ int fvgs_map_step(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics*
         FV_TRY(check_status(s, &retry));
         if (retry) {
             // the instance buffers grew; checkpoint slots follow capacity
-            FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H, cap));
+            FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H));
             continue;
         }
         s->has_map = true;

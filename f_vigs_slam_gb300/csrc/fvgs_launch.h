@@ -362,14 +362,11 @@ struct MapArgs {
     const float* obs_depth;  // P
     int W, H, ntx, nty;
     float bg[3];
-    const uint32_t* bucket_base;  // [T] exclusive bucket offsets (null with MAP_CAP256)
-    float4* sampled;              // [buckets][256] (T, accumulated colour)
     float* final_T;               // P
     uint32_t* n_contrib;          // P
     float* color;                 // 3P, incl. background
     float* depth;                 // P
     float* color_err;             // 3P
-    uint32_t* max_contrib;        // T
     float* delta2d;               // [N][16]: DeltaGaussian2D fields, n as u32 at 12
     float w_depth, w_dist;
 };
@@ -382,6 +379,7 @@ struct MapUpdateArgs {
     uint32_t cap;
     int n;
     const float* delta2d;
+    const uint32_t* counts;  // instances of each Gaussian in the step's binning (0: no gradient)
     const DevPose* pose;
     fvgs_intrinsics K;
     float lambda_iso, eta, beta1, beta2, eps;
@@ -391,11 +389,10 @@ struct MapUpdateArgs {
     CandState* cst;      // optional: n_cst candidate-list states, all stale once positions move
     int n_cst;
 };
-cudaError_t launch_map_forward(const MapArgs& a, bool cap, cudaStream_t s);
+cudaError_t launch_map_forward(const MapArgs& a, cudaStream_t s);
+// cap: only the first 256 entries of a tile's list receive gradients (MAP_CAP256).
 cudaError_t launch_map_backward(const MapArgs& a, bool cap, cudaStream_t s);
-cudaError_t launch_bucket_scan(const uint2* ranges, int T, uint32_t* bucket_base, uint32_t* total, cudaStream_t s);
-cudaError_t launch_map_update(const MapUpdateArgs& a, const DevStatus* st, cudaStream_t s);
-int map_cap_buckets();
+cudaError_t launch_map_update(const MapUpdateArgs& a, const DevStatus* st, int num_sms, cudaStream_t s);
 // Reduced-precision planes from the FP32 master planes (precision form).
 cudaError_t launch_pack_reduced(const float4* scale, const float4* rot, const float4* col, uint32_t n, uint4* sr,
                                 uint2* c, cudaStream_t s);

@@ -8,257 +8,255 @@
 // updateGaussiansParametersAdam_kernel (2722-2882).
 //
 // GPU structure:
-//  * forward: one CTA per 16x16 tile, Gaussian records staged in shared memory;
-//    checkpoints (T, accumulated colour) as one float4 per (bucket, pixel).
-//    With MAP_CAP256 only buckets 0..7 can receive gradients, so only those are
-//    checkpointed (tile*8 + b), and no bucket scan is needed.
-//  * backward: one CTA per tile; the tile's per-pixel forward results are
-//    staged once in shared memory and every warp runs the reference's
-//    lane-per-Gaussian pipeline over the 256 pixels, shuffling only the
-//    evolving state (T and the accumulated colour: 4 values, not 13);
+//  * forward and backward: every warp walks its tile's list for its own 8 x 4
+//    pixels (walk_list, as the tracking kernel), a lane per pixel.  The
+//    backward pass carries the pixel's T and accumulated colour along the list
+//    again, so the forward pass leaves no checkpoints; the reference's restart
+//    from a checkpoint every 32 list entries is the forward pass's state,
+//    carried beside.  A Gaussian's twelve sums are added over the warp by a
+//    butterfly and go to memory with one reduction of 12 lanes;
 //  * 2D->3D and Adam are fused: the 3D deltas never go to memory.
-#include "fvgs_device.cuh"
-#include "fvgs_launch.h"
+#include <algorithm>
+
+#include "track_tile.cuh"
 
 namespace fvgs {
 
-constexpr int kMPix = 256;
-constexpr int kMBatch = 256;
-constexpr int kCapBuckets = 8;
-constexpr float kMInv255 = 1.0f / 255.0f;
+constexpr int kMapCap = 256;  // list entries that receive gradients with MAP_CAP256
 
-template <bool CAP>
-__global__ void __launch_bounds__(kMPix) map_forward_kernel(MapArgs a) {
-    pdl_begin();
-    __shared__ float4 s0[kMBatch];
-    __shared__ float4 s1[kMBatch];
-    __shared__ float4 s2[kMBatch];
-    __shared__ uint32_t s_max;
-    const int tile = blockIdx.x;
-    const int tx = tile % a.ntx, ty = tile / a.ntx;
-    const int tid = threadIdx.x;
-    const int x = tx * 16 + (tid & 15), y = ty * 16 + (tid >> 4);
-    const bool inside = (x < a.W && y < a.H);
-    uint2 range = a.ranges[tile];
-    range.y = min(range.y, a.n_list);
-    const int n = range.y > range.x ? (int)(range.y - range.x) : 0;
-    const uint32_t base_slot = CAP ? (uint32_t)tile * kCapBuckets : a.bucket_base[tile];
-    const float xf = (float)x, yf = (float)y;
-    if (tid == 0) s_max = 0;
-    float T = 1.f, cr = 0.f, cg = 0.f, cb = 0.f, depth = 0.f;
-    uint32_t contributor = 0, last = 0;
-    bool done = !inside;
-    for (int base = 0; base < n; base += kMBatch) {
-        if (__syncthreads_and(done)) break;
-        const int li = base + tid;
-        if (li < n) {
-            const uint32_t g = a.indices[range.x + li];
-            const bool ok = g < a.n_gauss;  // zero opacity otherwise: never blends
-            float4 r0 = ok ? a.rec0[g] : make_float4(0.f, 0.f, 0.f, 0.f);
-            r0.w = log2_opacity(r0.w);  // staged as log2(opacity) for gauss_alpha
-            s0[tid] = r0;
-            s1[tid] = ok ? a.rec1[g] : make_float4(0.f, 0.f, 0.f, 0.f);
-            s2[tid] = ok ? a.rec2[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+// Two warps a CTA, each an 8 x 8 pixel quarter of a 16 x 16 tile, two pixels a
+// lane (rows y and y + 4): a staged Gaussian is read, and its sums are added
+// over the warp, once for 64 pixels.
+struct MapBlock {
+    int x0, y0, x, y[2], n;
+    uint32_t list0;
+    bool inside[2];
+    __device__ explicit MapBlock(const MapArgs& a) {
+        const int tile = blockIdx.x >> 1, quarter = (blockIdx.x & 1) * 2 + (threadIdx.x >> 5);
+        const int lane = threadIdx.x & 31;
+        x0 = (tile % a.ntx) * 16 + (quarter & 1) * 8;
+        y0 = (tile / a.ntx) * 16 + (quarter >> 1) * 8;
+        x = x0 + (lane & 7);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            y[k] = y0 + (lane >> 3) + 4 * k;
+            inside[k] = x < a.W && y[k] < a.H;
         }
-        __syncthreads();
-        if (!done) {
-            const int cnt = min(kMBatch, n - base);
-            for (int j = 0; j < cnt; ++j) {
-                const int gi = base + j;
-                if ((gi & 31) == 0 && (!CAP || gi < 32 * kCapBuckets))
-                    a.sampled[(size_t)(base_slot + gi / 32) * kMPix + tid] = make_float4(T, cr, cg, cb);
-                ++contributor;
-                const float4 r0 = s0[j];
-                const float4 r1 = s1[j];
-                const float dx = xf - r0.x, dy = yf - r0.y;
-                float dl0, dl1;
-                const float v = conic_form(r1.x, r1.y, r1.z, dx, dy, dl0, dl1);
-                const float alpha = gauss_alpha(r0.w, v);
-                if (alpha < kMInv255 || v <= 0.0f) continue;
-                const float4 r2 = s2[j];
-                cr += T * alpha * r2.y;
-                cg += T * alpha * r2.z;
-                cb += T * alpha * r2.w;
-                const float test_T = T * (1.0f - alpha);
-                if (T > 0.5f && test_T <= 0.5f) depth = r0.z + r1.w * dx + r2.x * dy;
-                T = test_T;
-                last = contributor;
-                if (test_T < 0.0001f) {
-                    done = true;
-                    break;
+        uint2 range = a.ranges[tile];
+        range.y = min(range.y, a.n_list);
+        list0 = range.x;
+        n = range.y > range.x ? (int)(range.y - range.x) : 0;
+    }
+};
+
+// Forward pass.  What bounds it: issue; 1 M Gaussians, 1280x720: 125 us, before
+// (a CTA per tile, every list entry evaluated by every pixel, checkpoints)
+// 187.
+__global__ void __launch_bounds__(64) map_forward_kernel(MapArgs a) {
+    pdl_begin();
+    __shared__ WarpStage<0> stage[2];
+    WarpStage<0>& ws = stage[threadIdx.x >> 5];
+    const MapBlock blk(a);
+    const float xf = (float)blk.x;
+    float T[2], cr[2], cg[2], cb[2], depth[2];
+    uint32_t last[2];
+    int last_j[2];  // staged slot of the last blended Gaussian of this round
+    bool end[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        T[k] = 1.f;
+        cr[k] = cg[k] = cb[k] = depth[k] = 0.f;
+        last[k] = 0;
+        last_j[k] = -1;
+        end[k] = !blk.inside[k];
+    }
+    bool done = end[0] && end[1];
+    auto blend = [&](int j, const float4& rA, const float4& rB, float dxm, float dy0, float, float, float v0,
+                     float raw0) {
+        const float dy1 = rA.y - (float)blk.y[1];
+        float q0, q1;
+        const float v1 = conic_form(rA.z, rA.w, rB.x, dxm, dy1, q0, q1);
+        const float raw1 = gauss_weight(rB.z, v1);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float v = k ? v1 : v0, dym = k ? dy1 : dy0;
+            const float alpha = fminf(0.99f, k ? raw1 : raw0);
+            if (!(end[k] || v > rB.y || v <= 0.0f || alpha < kInv255)) {
+                const float4 rC = ws.C[j];
+                cr[k] += T[k] * alpha * rC.z;
+                cg[k] += T[k] * alpha * rC.w;
+                cb[k] += T[k] * alpha * ws.E[j].x;
+                const float test_T = T[k] * (1.0f - alpha);
+                if (T[k] > 0.5f && test_T <= 0.5f) {
+                    const float dx = -dxm, dy = -dym;  // pixel - mean
+                    depth[k] = rB.w + rC.x * dx + rC.y * dy;
+                }
+                T[k] = test_T;
+                last_j[k] = j;
+                if (test_T < 0.0001f) end[k] = true;
+            }
+        }
+        done = end[0] && end[1];
+    };
+    auto round_end = [&]() {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (last_j[k] >= 0) last[k] = (uint32_t)__float_as_int(ws.E[last_j[k]].y) + 1u;
+            last_j[k] = -1;
+        }
+    };
+    walk_list<false, kMasksNone, kStageNone, 8>(a, ws, blk.list0, blk.n, (float)blk.x0, (float)blk.y0, xf,
+                                                (float)blk.y[0], done, blend, round_end);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (!blk.inside[k]) continue;
+        const size_t p = (size_t)blk.y[k] * a.W + blk.x;
+        a.final_T[p] = T[k];
+        a.n_contrib[p] = last[k];
+        cr[k] += T[k] * a.bg[0];
+        cg[k] += T[k] * a.bg[1];
+        cb[k] += T[k] * a.bg[2];
+        a.color[3 * p] = cr[k];
+        a.color[3 * p + 1] = cg[k];
+        a.color[3 * p + 2] = cb[k];
+        a.depth[p] = depth[k];
+        a.color_err[3 * p] = cr[k] - a.obs_rgb[3 * p];
+        a.color_err[3 * p + 1] = cg[k] - a.obs_rgb[3 * p + 1];
+        a.color_err[3 * p + 2] = cb[k] - a.obs_rgb[3 * p + 2];
+    }
+}
+
+// Sum of 12 values over the warp: the lane whose bit 0 is clear and whose
+// slot() is below 12 returns the sum of v[slot()].
+struct WarpSum12 {
+    // bit 4 picks a half, bit 3 a quarter, bits 2 and 1 one of three
+    static __device__ __forceinline__ int slot(int lane) {
+        const int k = ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+        return (lane & 1) || k > 2 ? 12 : ((lane >> 4) & 1) * 6 + ((lane >> 3) & 1) * 3 + k;
+    }
+    static __device__ __forceinline__ float run(const float (&v)[12], int lane) {
+        float a[6], b[4], c[2];
+        const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4, h1 = lane & 2;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) a[k] = (h4 ? v[k + 6] : v[k]) + __shfl_xor_sync(kFullMask, h4 ? v[k] : v[k + 6], 16);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) b[k] = (h3 ? a[k + 3] : a[k]) + __shfl_xor_sync(kFullMask, h3 ? a[k] : a[k + 3], 8);
+        b[3] = 0.f;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) c[k] = (h2 ? b[k + 2] : b[k]) + __shfl_xor_sync(kFullMask, h2 ? b[k] : b[k + 2], 4);
+        const float d = (h1 ? c[1] : c[0]) + __shfl_xor_sync(kFullMask, h1 ? c[0] : c[1], 2);
+        return d + __shfl_xor_sync(kFullMask, d, 1);
+    }
+};
+
+// Backward pass.  n_max: list entries that receive gradients.  What bounds it:
+// issue -- about 60 instructions of gradient a pixel and 55 of warp sum for a
+// visited block and Gaussian (one pixel a lane: 437 us).  1 M Gaussians, 1280x720: 360 us, before (a lane per
+// Gaussian, pixels passed from lane to lane in list order, one step per pixel
+// and bucket of 32 entries whether they meet or not) 652.
+__global__ void __launch_bounds__(64, 8) map_backward_kernel(MapArgs a, int n_max) {
+    pdl_begin();
+    __shared__ WarpStage<0> stage[2];
+    WarpStage<0>& ws = stage[threadIdx.x >> 5];
+    const MapBlock blk(a);
+    const int lane = threadIdx.x & 31, slot = WarpSum12::slot(lane);
+    const float xf = (float)blk.x;
+    uint32_t nc[2] = {0u, 0u};
+    float4 pc[2], pe[2];             // final colour and depth; colour error, observed depth
+    float T[2], a0[2], a1[2], a2[2];  // this pass's state
+    float Tf[2], f0[2], f1[2], f2[2];  // the forward pass's state
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        pc[k] = pe[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (blk.inside[k]) {
+            const size_t p = (size_t)blk.y[k] * a.W + blk.x;
+            nc[k] = a.n_contrib[p];
+            pc[k] = make_float4(a.color[3 * p], a.color[3 * p + 1], a.color[3 * p + 2], a.depth[p]);
+            pe[k] = make_float4(a.color_err[3 * p], a.color_err[3 * p + 1], a.color_err[3 * p + 2], a.obs_depth[p]);
+        }
+        T[k] = Tf[k] = 1.f;
+        a0[k] = a1[k] = a2[k] = f0[k] = f1[k] = f2[k] = 0.f;
+    }
+    const uint32_t nc_max = max(nc[0], nc[1]);
+    const int n = min(min(blk.n, n_max), (int)__reduce_max_sync(kFullMask, nc_max));
+    const float w_depth = a.w_depth, w_dist = a.w_dist;
+    bool done = nc_max == 0;
+    auto grad = [&](int j, const float4& rA, const float4& rB, float dx, float dy0, float l00, float l01, float v0,
+                    float raw0) {
+        const float2 rE = ws.E[j];
+        const float dy1 = rA.y - (float)blk.y[1];
+        float l10, l11;
+        const float v1 = conic_form(rA.z, rA.w, rB.x, dx, dy1, l10, l11);
+        const float al[2] = {fminf(0.99f, raw0), fminf(0.99f, gauss_weight(rB.z, v1))};
+        const uint32_t li = (uint32_t)__float_as_int(rE.y);
+        // (the entry that fills up an odd count has v > rB.y, whatever its list index)
+        const bool on[2] = {li < nc[0] && !(v0 > rB.y || al[0] < kInv255), li < nc[1] && !(v1 > rB.y || al[1] < kInv255)};
+        const uint32_t hit0 = __ballot_sync(kFullMask, on[0]), hit1 = __ballot_sync(kFullMask, on[1]);
+        if (rB.y != -INFINITY && li >= nc_max) done = true;
+        if ((hit0 | hit1) == 0u) return;
+        const float4 rC = ws.C[j];
+        float s[12];
+#pragma unroll
+        for (int k = 0; k < 12; ++k) s[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (on[k]) {
+                const float alpha = al[k], dy = k ? dy1 : dy0;
+                float d0 = rC.z * T[k], d1 = rC.w * T[k], d2 = rE.x * T[k];
+                a0[k] += d0 * alpha;
+                a1[k] += d1 * alpha;
+                a2[k] += d2 * alpha;
+                const float inv1m = rcp_approx(1.0f - alpha);
+                d0 = (d0 - (pc[k].x - a0[k]) * inv1m) * -pe[k].x;
+                d1 = (d1 - (pc[k].y - a1[k]) * inv1m) * -pe[k].y;
+                d2 = (d2 - (pc[k].z - a2[k]) * inv1m) * -pe[k].z;
+                const float aG = alpha * (d0 + d1 + d2);
+                const float aT = alpha * T[k];
+                const float haG = 0.5f * aG;
+                const float test_T = T[k] * (1.0f - alpha);
+                const float di = rB.w + dx * rC.x + dy * rC.y;
+                float dc = w_dist * alpha * T[k] * (di - pc[k].w);
+                if (T[k] > 0.5f && test_T <= 0.5f) {
+                    const float derr = (pe[k].w > 0.1f) ? (pc[k].w - pe[k].w) : 0.0f;
+                    dc += w_depth * derr;
+                }
+                s[0] -= aG * (k ? l10 : l00) + dc * rC.x;
+                s[1] -= aG * (k ? l11 : l01) + dc * rC.y;
+                s[2] -= haG * dx * dx;
+                s[3] -= haG * dx * dy;
+                s[4] -= haG * dy * dy;
+                s[5] -= aT * pe[k].x;
+                s[6] -= aT * pe[k].y;
+                s[7] -= aT * pe[k].z;
+                s[8] -= dc;
+                s[9] -= aG;
+                s[10] -= dc * dx;
+                s[11] -= dc * dy;
+                T[k] = test_T;
+                if ((k ? v1 : v0) > 0.0f) {
+                    f0[k] += Tf[k] * alpha * rC.z;
+                    f1[k] += Tf[k] * alpha * rC.w;
+                    f2[k] += Tf[k] * alpha * rE.x;
+                    Tf[k] *= 1.0f - alpha;
                 }
             }
         }
-    }
-    if (inside) {
-        const size_t p = (size_t)y * a.W + x;
-        a.final_T[p] = T;
-        a.n_contrib[p] = last;
-        cr += T * a.bg[0];
-        cg += T * a.bg[1];
-        cb += T * a.bg[2];
-        a.color[3 * p] = cr;
-        a.color[3 * p + 1] = cg;
-        a.color[3 * p + 2] = cb;
-        a.depth[p] = depth;
-        a.color_err[3 * p] = cr - a.obs_rgb[3 * p];
-        a.color_err[3 * p + 1] = cg - a.obs_rgb[3 * p + 1];
-        a.color_err[3 * p + 2] = cb - a.obs_rgb[3 * p + 2];
-    }
-    __syncthreads();
-    if (last) atomicMax(&s_max, last);
-    __syncthreads();
-    if (tid == 0) a.max_contrib[tile] = s_max;
-}
-
-template <bool CAP>
-__global__ void __launch_bounds__(kMPix, 4) map_backward_kernel(MapArgs a) {
-    pdl_begin();
-    __shared__ float4 s_pc[kMPix];  // final colour (incl. background), median depth
-    __shared__ float4 s_pe[kMPix];  // colour error, observed depth
-    __shared__ uint32_t s_nc[kMPix];
-    __shared__ uint16_t s_act[kMPix / 32][kMPix];  // per warp: the pixels its bucket can reach
-    const int tile = blockIdx.x;
-    const int tx = tile % a.ntx, ty = tile / a.ntx;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    uint2 range = a.ranges[tile];
-    range.y = min(range.y, a.n_list);
-    const uint32_t n = range.y > range.x ? range.y - range.x : 0u;
-    const uint32_t maxc = a.max_contrib[tile];
-    uint32_t nb = (n + 31) / 32;
-    if (CAP) nb = min(nb, (uint32_t)kCapBuckets);
-    if (nb == 0 || maxc == 0) return;
-    {
-        const int px = tx * 16 + (tid & 15), py = ty * 16 + (tid >> 4);
-        if (px < a.W && py < a.H) {
-            const size_t p = (size_t)py * a.W + px;
-            s_pc[tid] = make_float4(a.color[3 * p], a.color[3 * p + 1], a.color[3 * p + 2], a.depth[p]);
-            s_pe[tid] = make_float4(a.color_err[3 * p], a.color_err[3 * p + 1], a.color_err[3 * p + 2],
-                                    a.obs_depth[p]);
-            s_nc[tid] = a.n_contrib[p];
-        } else {
-            s_nc[tid] = 0;  // out-of-image pixels are never processed
+        const float sum = WarpSum12::run(s, lane);
+        float* D = a.delta2d + (size_t)ws.G[j] * 16;
+        if (slot < 12) atomicAdd(D + slot, sum);
+        if (lane == 31) atomicAdd(reinterpret_cast<uint32_t*>(D + 12), (uint32_t)(__popc(hit0) + __popc(hit1)));
+    };
+    auto round_end = [&]() {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            T[k] = Tf[k];
+            a0[k] = f0[k];
+            a1[k] = f1[k];
+            a2[k] = f2[k];
         }
-    }
-    __syncthreads();
-    const uint32_t base_slot = CAP ? (uint32_t)tile * kCapBuckets : a.bucket_base[tile];
-    const float w_depth = a.w_depth, w_dist = a.w_dist;
-    for (uint32_t b = warp; b < nb; b += kMPix / 32) {
-        if (b * 32 >= maxc) break;
-        const uint32_t j = b * 32 + lane;
-        bool valid_splat = j < n && (!CAP || j < 32u * kCapBuckets);
-        float4 r0 = make_float4(0, 0, 0, 0), r1 = r0, r2 = r0;
-        uint32_t gid = 0;
-        if (valid_splat) {
-            gid = a.indices[range.x + j];
-            valid_splat = gid < a.n_gauss;
-        }
-        if (valid_splat) {
-            r0 = a.rec0[gid];
-            r1 = a.rec1[gid];
-            r2 = a.rec2[gid];
-        }
-        const float lo2 = log2_opacity(r0.w);  // the forward pass's alpha from log2(opacity)
-        float dmx = 0.f, dmy = 0.f, dix = 0.f, diy = 0.f, diz = 0.f, dcr = 0.f, dcg = 0.f, dcb = 0.f;
-        float dz = 0.f, dal = 0.f, dpx = 0.f, dpy = 0.f;
-        uint32_t dn = 0;
-        float T = 0.f, a0 = 0.f, a1 = 0.f, a2 = 0.f;
-        const float4* samp = a.sampled + (size_t)(base_slot + b) * kMPix;
-        // Only pixels whose contributor count exceeds the bucket's first list
-        // position can receive anything from it; the pipeline walks those, in
-        // pixel order (each starts from its own checkpoint, so skipping the
-        // others changes no sum).
-        int n_act = 0;
-        for (int c = 0; c < kMPix; c += 32) {
-            const bool act = s_nc[c + lane] > b * 32;
-            const unsigned m = __ballot_sync(kFullMask, act);
-            if (act) s_act[warp][n_act + __popc(m & lanemask_lt())] = (uint16_t)(c + lane);
-            n_act += __popc(m);
-        }
-        __syncwarp();
-        for (int i = 0; i < n_act + 31; ++i) {
-            T = __shfl_up_sync(kFullMask, T, 1);
-            a0 = __shfl_up_sync(kFullMask, a0, 1);
-            a1 = __shfl_up_sync(kFullMask, a1, 1);
-            a2 = __shfl_up_sync(kFullMask, a2, 1);
-            const int pos = i - lane;
-            if (!valid_splat || pos < 0 || pos >= n_act) continue;
-            const int idx = s_act[warp][pos];
-            const uint32_t nc = s_nc[idx];
-            if (lane == 0 && nc != 0) {
-                const float4 sv = samp[idx];
-                T = sv.x;
-                a0 = sv.y;
-                a1 = sv.z;
-                a2 = sv.w;
-            }
-            if (j >= nc) continue;
-            const float pxf = (float)(tx * 16 + (idx & 15)), pyf = (float)(ty * 16 + (idx >> 4));
-            const float dx = r0.x - pxf, dy = r0.y - pyf;
-            float dl0, dl1;  // the forward pass's conic form ((dx, dy) negated: same value)
-            const float v = conic_form(r1.x, r1.y, r1.z, dx, dy, dl0, dl1);
-            const float alpha = gauss_alpha(lo2, v);
-            if (alpha < kMInv255) continue;
-            const float4 pc = s_pc[idx];
-            const float4 pe = s_pe[idx];
-            float d0 = r2.y * T, d1 = r2.z * T, d2 = r2.w * T;
-            a0 += d0 * alpha;
-            a1 += d1 * alpha;
-            a2 += d2 * alpha;
-            const float inv1m = rcp_approx(1.0f - alpha);
-            d0 = (d0 - (pc.x - a0) * inv1m) * -pe.x;
-            d1 = (d1 - (pc.y - a1) * inv1m) * -pe.y;
-            d2 = (d2 - (pc.z - a2) * inv1m) * -pe.z;
-            const float aG = alpha * (d0 + d1 + d2);
-            ++dn;
-            const float aT = alpha * T;
-            dcr -= aT * pe.x;
-            dcg -= aT * pe.y;
-            dcb -= aT * pe.z;
-            dal -= aG;
-            dmx -= aG * dl0;
-            dmy -= aG * dl1;
-            const float haG = 0.5f * aG;
-            dix -= haG * dx * dx;
-            diy -= haG * dx * dy;
-            diz -= haG * dy * dy;
-            const float test_T = T * (1.0f - alpha);
-            const float phx = r1.w, phy = r2.x;
-            if (T > 0.5f && test_T <= 0.5f) {
-                const float derr = (pe.w > 0.1f) ? (pc.w - pe.w) : 0.0f;
-                const float wde = w_depth * derr;
-                dz -= wde;
-                dmx -= wde * phx;
-                dmy -= wde * phy;
-                dpx -= wde * dx;
-                dpy -= wde * dy;
-            }
-            const float di = r0.z + dx * phx + dy * phy;
-            const float dc = w_dist * alpha * T * (di - pc.w);
-            dz -= dc;
-            dmx -= dc * phx;
-            dmy -= dc * phy;
-            dpx -= dc * dx;
-            dpy -= dc * dy;
-            T = test_T;
-        }
-        if (valid_splat && dn > 0) {
-            float* D = a.delta2d + (size_t)gid * 16;
-            atomicAdd(D + 0, dmx);
-            atomicAdd(D + 1, dmy);
-            atomicAdd(D + 2, dix);
-            atomicAdd(D + 3, diy);
-            atomicAdd(D + 4, diz);
-            atomicAdd(D + 5, dcr);
-            atomicAdd(D + 6, dcg);
-            atomicAdd(D + 7, dcb);
-            atomicAdd(D + 8, dz);
-            atomicAdd(D + 9, dal);
-            atomicAdd(D + 10, dpx);
-            atomicAdd(D + 11, dpy);
-            atomicAdd(reinterpret_cast<uint32_t*>(D + 12), dn);
-        }
-    }
+    };
+    walk_list<false, kMasksSecond, kStageIndex, 8>(a, ws, blk.list0, n, (float)blk.x0, (float)blk.y0, xf,
+                                                   (float)blk.y[0], done, grad, round_end);
 }
 
 // ----------------------- 2D -> 3D chain rule + Adam ------------------------
@@ -297,24 +295,11 @@ __device__ __forceinline__ float adam_step(float& m, float& v, float g, float et
     return eta * (b1t * m) * rsqrtf(b2t * v + eps);
 }
 
-__global__ void __launch_bounds__(256) map_update_kernel(MapUpdateArgs a, const DevStatus* st) {
-    pdl_begin();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.n_cst && a.cst) a.cst[i].valid = 0;
-    if (i >= a.n) return;
-    // An instance overflow leaves the binning incomplete; the host re-runs the
-    // step with larger buffers, so the parameters must stay untouched.
-    if (st->flags & kErrOverflow) return;
+// One Gaussian with a gradient (nn contributing pixels).
+__device__ __forceinline__ void update_one(const MapUpdateArgs& a, int i) {
     const float4* D4 = reinterpret_cast<const float4*>(a.delta2d + (size_t)i * 16);
-    // the contributor count first: most of a large map has no gradient, and
-    // then only this one sector of the record is read
-    const float4 q3 = D4[3];
-    const uint32_t nn = __float_as_uint(q3.x);
-    if (nn == 0) {
-        if (a.dbg_delta3d)
-            for (int k = 0; k < 16; ++k) a.dbg_delta3d[(size_t)i * 16 + k] = 0.f;
-        return;
-    }
+    const uint32_t nn = __float_as_uint(D4[3].x);
+    if (nn == 0) return;
     const float4 q0 = D4[0], q1 = D4[1], q2 = D4[2];
     const float d_mean[2] = {q0.x, q0.y};
     const float d_inv[3] = {q0.z, q0.w, q1.x};
@@ -589,69 +574,67 @@ __global__ void __launch_bounds__(256) map_update_kernel(MapUpdateArgs a, const 
     S[8 * NN + i] = mal;
 }
 
-// Exclusive scan of per-tile bucket counts ceil(n_t/32) (one CTA).
-__global__ void __launch_bounds__(1024) bucket_scan_kernel(const uint2* ranges, int T, uint32_t* bucket_base,
-                                                           uint32_t* total) {
+// A CTA takes kUpdThreads * per Gaussians: first their instance counts, the
+// ones with instances queued in shared memory, then the queue with full warps
+// -- most of a large map is out of view, so in index order only a few lanes
+// of a warp would run the chain rule and Adam.  per spreads a small map over
+// all SMs (1) and gives a large one full queues (8).  What bounds it: the
+// latency of the queued Gaussians' state (464 bytes each).  1 M Gaussians, 86 k
+// in view: 33 us, before (a thread per Gaussian, its gradient count read from
+// the 64-byte record) 74.
+constexpr int kUpdThreads = 256, kUpdMost = 8;
+__global__ void __launch_bounds__(kUpdThreads) map_update_kernel(MapUpdateArgs a, int per, const DevStatus* st) {
     pdl_begin();
-    __shared__ uint32_t s_w[32];
-    __shared__ uint32_t s_carry;
-    if (threadIdx.x == 0) s_carry = 0;
+    __shared__ uint32_t q_i[kUpdThreads * kUpdMost];
+    __shared__ int q_n;
+    const int t = threadIdx.x, lane = t & 31;
+    if (blockIdx.x == 0 && t < a.n_cst && a.cst) a.cst[t].valid = 0;
+    // An instance overflow leaves the binning incomplete; the host re-runs the
+    // step with larger buffers, so the parameters must stay untouched.
+    if (st->flags & kErrOverflow) return;
+    if (t == 0) q_n = 0;
     __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int base = 0; base < T; base += 1024) {
-        const int t = base + threadIdx.x;
-        uint32_t c = 0;
-        if (t < T) c = (ranges[t].y - ranges[t].x + 31) / 32;
-        uint32_t incl = c;
+    const int base = blockIdx.x * kUpdThreads * per;
+    uint32_t c[kUpdMost];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) s_w[w] = incl;
-        __syncthreads();
-        if (w == 0) {
-            const uint32_t v = s_w[lane];
-            uint32_t vi = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(kFullMask, vi, o);
-                if (lane >= o) vi += y;
-            }
-            s_w[lane] = vi - v;
-        }
-        __syncthreads();
-        const uint32_t carry = s_carry;
-        if (t < T) bucket_base[t] = carry + s_w[w] + incl - c;
-        __syncthreads();
-        if (threadIdx.x == 1023) s_carry = carry + s_w[w] + incl;
-        __syncthreads();
+    for (int k = 0; k < kUpdMost; ++k) {
+        const int i = base + k * kUpdThreads + t;
+        c[k] = k < per && i < a.n ? a.counts[i] : 0u;
     }
-    if (threadIdx.x == 0) *total = s_carry;
+#pragma unroll
+    for (int k = 0; k < kUpdMost; ++k) {
+        const int i = base + k * kUpdThreads + t;
+        const uint32_t bal = __ballot_sync(kFullMask, c[k] != 0u);
+        if (bal) {
+            int slot = 0;
+            if (lane == 0) slot = atomicAdd(&q_n, __popc(bal));
+            slot = __shfl_sync(kFullMask, slot, 0) + __popc(bal & lanemask_lt());
+            if (c[k]) q_i[slot] = (uint32_t)i;
+        }
+        if (a.dbg_delta3d && k < per && i < a.n)
+            for (int w = 0; w < 16; ++w) a.dbg_delta3d[(size_t)i * 16 + w] = 0.f;
+    }
+    __syncthreads();
+    const int n = q_n;
+    for (int k = t; k < n; k += kUpdThreads) update_one(a, (int)q_i[k]);
 }
 
-cudaError_t launch_map_forward(const MapArgs& a, bool cap, cudaStream_t s) {
-    const int T = a.ntx * a.nty;
-    if (cap) return launch_chained(map_forward_kernel<true>, dim3(T), dim3(kMPix), 0, s, a);
-    return launch_chained(map_forward_kernel<false>, dim3(T), dim3(kMPix), 0, s, a);
+cudaError_t launch_map_forward(const MapArgs& a, cudaStream_t s) {
+    return launch_chained(map_forward_kernel, dim3(2 * a.ntx * a.nty), dim3(64), 0, s, a);
 }
 
 cudaError_t launch_map_backward(const MapArgs& a, bool cap, cudaStream_t s) {
-    const int T = a.ntx * a.nty;
-    if (cap) return launch_chained(map_backward_kernel<true>, dim3(T), dim3(kMPix), 0, s, a);
-    return launch_chained(map_backward_kernel<false>, dim3(T), dim3(kMPix), 0, s, a);
+    return launch_chained(map_backward_kernel, dim3(2 * a.ntx * a.nty), dim3(64), 0, s, a,
+                          cap ? kMapCap : 0x7fffffff);
 }
 
-cudaError_t launch_bucket_scan(const uint2* ranges, int T, uint32_t* bucket_base, uint32_t* total, cudaStream_t s) {
-    return launch_chained(bucket_scan_kernel, dim3(1), dim3(1024), 0, s, ranges, T, bucket_base, total);
-}
-
-cudaError_t launch_map_update(const MapUpdateArgs& a, const DevStatus* st, cudaStream_t s) {
+cudaError_t launch_map_update(const MapUpdateArgs& a, const DevStatus* st, int num_sms, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
-    return launch_chained(map_update_kernel, dim3((a.n + 255) / 256), dim3(256), 0, s, a, st);
+    // two CTAs an SM: as many Gaussians each as fill them once
+    const int per = std::max(1, std::min(kUpdMost, a.n / (2 * num_sms * kUpdThreads)));
+    const int chunk = per * kUpdThreads;
+    return launch_chained(map_update_kernel, dim3((a.n + chunk - 1) / chunk), dim3(kUpdThreads), 0, s, a, per, st);
 }
-
-int map_cap_buckets() { return kCapBuckets; }
 
 __global__ void pack_reduced_kernel(const float4* __restrict__ scale, const float4* __restrict__ rot,
                                     const float4* __restrict__ col, uint32_t n, uint4* __restrict__ sr,

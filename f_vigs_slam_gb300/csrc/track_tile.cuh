@@ -142,7 +142,7 @@ __device__ __forceinline__ void load_ref_record(const TrackArgs& a, uint32_t g, 
     r2 = make_float4(ph.y, a.ref_col[3 * (size_t)g], a.ref_col[3 * (size_t)g + 1], a.ref_col[3 * (size_t)g + 2]);
 }
 
-// Rejection of a Gaussian by a warp's 8 x 4 pixel block, once per staged
+// Rejection of a Gaussian by a warp's 8 x ROWS pixel block, once per staged
 // Gaussian.  A pixel skips a Gaussian when v > vreject (alpha < 1/255, both
 // passes) or, in the forward pass only, when v <= 0.  If the extremes of v
 // over the block prove one of these for every pixel -- kRejectAlpha: min v >
@@ -163,12 +163,13 @@ __device__ __forceinline__ void load_ref_record(const TrackArgs& a, uint32_t g, 
 // minimum where it is convex, else a maximum).  The stationary points come
 // from rcp.approx: one ulp off changes v by 1e-14 of its terms.
 constexpr uint32_t kRejectAlpha = 1u, kRejectSign = 2u;
+template <int ROWS = 4>
 __device__ __forceinline__ uint32_t block_reject(float u, float v, float ca, float cb, float cc, float vrej, float x0,
                                                  float y0) {
     if (vrej == -INFINITY) return kRejectAlpha;  // zero opacity: alpha is 0 everywhere
     if (!(isfinite(u) && isfinite(v) && isfinite(ca) && isfinite(cb) && isfinite(cc) && isfinite(vrej))) return 0u;
     const float dxlo = u - (x0 + 7.0f), dxhi = u - x0;
-    const float dylo = v - (y0 + 3.0f), dyhi = v - y0;
+    const float dylo = v - (y0 + (float)(ROWS - 1)), dyhi = v - y0;
     const float mx = fmaxf(fabsf(dxlo), fabsf(dxhi)), my = fmaxf(fabsf(dylo), fabsf(dyhi));
     const float margin = 1e-5f * (fabsf(ca) * mx * mx + 2.0f * fabsf(cb) * mx * my + fabsf(cc) * my * my) + 1e-3f;
     auto q = [&](float dx, float dy) { return ca * dx * dx + 2.0f * cb * dx * dy + cc * dy * dy; };
@@ -218,7 +219,7 @@ struct WarpStage {
 };
 
 // What a staging round stores besides the blending record.
-enum StageExtra { kStageNone = 0, kStageRay = 1, kStageDeriv = 2 };
+enum StageExtra { kStageNone = 0, kStageRay = 1, kStageDeriv = 2, kStageIndex = 3 };
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -230,7 +231,7 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
-// Walk the first n entries of the tile's list for one warp's 8 x 4 pixel
+// Walk the first n entries of the tile's list for one warp's 8 x ROWS pixel
 // block with corner (x0, y0), front to back, until every lane is done.  The
 // warp stages kRound entries at a time on its own -- each lane takes one
 // entry, drops it when the block cannot see it, and the survivors are
@@ -242,9 +243,10 @@ __device__ __forceinline__ void cp_async_wait() {
 // MASKS: this walk's use of the kept survivors of the second pass (the
 // reference Jacobian's rejection test costs more than the rest of its staging,
 // and the first pass has both answers at hand).
-enum WalkMasks { kMasksNone = 0, kMasksKeep = 1, kMasksUse = 2 };
-template <bool REF_LAYOUT, int MASKS, int STAGE, int NX, class Pair, class RoundEnd>
-__device__ __forceinline__ void walk_list(const TrackArgs& a, WarpStage<NX>& ws, uint32_t list0, int n, float x0,
+// kMasksSecond: the second pass's survivors, without masks from a first.
+enum WalkMasks { kMasksNone = 0, kMasksKeep = 1, kMasksUse = 2, kMasksSecond = 3 };
+template <bool REF_LAYOUT, int MASKS, int STAGE, int ROWS = 4, class Args, int NX, class Pair, class RoundEnd>
+__device__ __forceinline__ void walk_list(const Args& a, WarpStage<NX>& ws, uint32_t list0, int n, float x0,
                                           float y0, float xf, float yf, bool& done, Pair&& pair,
                                           RoundEnd&& round_end) {
     const int lane = threadIdx.x & 31;
@@ -285,8 +287,8 @@ __device__ __forceinline__ void walk_list(const TrackArgs& a, WarpStage<NX>& ws,
             if (MASKS == kMasksUse && base < kRound * kMaskRounds)
                 keep = (ws.M[base / kRound] >> lane) & 1u;
             else {
-                rej = block_reject(r0.x, r0.y, r1.x, r1.y, r1.z, vrej, x0, y0);
-                keep = MASKS == kMasksUse ? !(rej & kRejectAlpha) : rej == 0u;
+                rej = block_reject<ROWS>(r0.x, r0.y, r1.x, r1.y, r1.z, vrej, x0, y0);
+                keep = MASKS >= kMasksUse ? !(rej & kRejectAlpha) : rej == 0u;
             }
         }
         if constexpr (MASKS == kMasksKeep) {
@@ -301,7 +303,7 @@ __device__ __forceinline__ void walk_list(const TrackArgs& a, WarpStage<NX>& ws,
             ws.B[pos] = make_float4(r1.z, vrej, lo2, r0.z);
             ws.C[pos] = make_float4(r1.w, r2.x, r2.y, r2.z);
             ws.E[pos] = make_float2(r2.w, __int_as_float(li));
-            if constexpr (STAGE == kStageDeriv) ws.G[pos] = g;
+            if constexpr (STAGE == kStageDeriv || STAGE == kStageIndex) ws.G[pos] = g;
             if constexpr (STAGE == kStageRay) {
                 const float rgx = (r0.x - a.K.cx) * __frcp_rn(a.K.fx), rgy = (r0.y - a.K.cy) * __frcp_rn(a.K.fy);
                 ws.X[pos][0] = make_float4(rgx, rgy, -a.K.fx * rgx, -a.K.fy * rgy);

@@ -107,3 +107,34 @@ def test_map_step_parity_vga_50k(oracle, fvgs_lib, quirks):
         e = rel_err(g["delta3d"][same][:, cols], o.delta3d[same][:, cols])
         print("delta3d", name, e)
         assert e <= GRAD_RTOL, (name, e)
+
+
+@pytest.mark.parametrize("quirks", [0x4 | 0x8, 0x0], ids=["ref", "intended"])
+@pytest.mark.parametrize("n", [1, 33, 257, 300])
+@pytest.mark.parametrize("size", [(16, 16), (21, 13), (9, 5)])
+def test_map_step_list_and_block_edges(oracle, fvgs_lib, size, n, quirks):
+    """Lists around a warp's round of 32 entries and the 256-entry cap, and 8 x 8
+    pixel blocks partly or wholly outside the image."""
+    W, H = size
+    K = (30.0, 30.0, (W - 1) / 2.0, (H - 1) / 2.0)
+    rng = np.random.default_rng(100 * n + W)
+    scene = S.cam_box(n, seed=n)
+    scene.positions[:, :2] = rng.uniform(-0.1, 0.1, (n, 2)) * scene.positions[:, 2:]
+    scene.scales[:] = rng.uniform(0.2, 0.6, (n, 3))
+    scene.opacities[:] *= 0.2  # long lists before a pixel is opaque
+    P = oracle.default_params(quirks)
+    pose = (np.zeros(3, np.float32), S.IDENTITY_Q)
+    rgb, d, gx, gy = make_frame(oracle, scene, S.perturb(pose, 0.3, 0.5, rng), K, W, H, P)
+    b = oracle.prepare(scene, pose, K, W, H, P)
+    o = oracle.map_step(scene, b, rgb, d, pose, K, W, H, P, ETA)
+    with fvgs_lib.Session(n, W, H, fvgs_lib.default_params(quirks)) as s:
+        s.upload(scene)
+        s.set_frame(0, rgb, d, gx, gy)
+        s.map_step(pose, K, ETA)
+        g = s.download_map_state(W, H)
+    same = g["delta2d"][:, 12] == o.delta2d[:, 12]
+    assert same.mean() >= 0.97, same.mean()
+    assert np.mean(g["n_contrib"] == o.n_contrib.reshape(H, W)) >= 0.97
+    for name, cols in GROUPS_2D.items():
+        e = rel_err(g["delta2d"][same][:, cols], o.delta2d[same][:, cols])
+        assert e <= GRAD_RTOL, (name, e)
