@@ -212,10 +212,14 @@ __device__ __forceinline__ float reject_bound(float o, float log2_o) {
     return b + 1e-3f + 1e-4f * fabsf(b);
 }
 
-__device__ __forceinline__ float gauss_weight(float log2_o, float v) {
+__device__ __forceinline__ float ex2_approx(float x) {
     float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmaf_rn(v, -0.72134752044448170368f, log2_o)));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x));
     return e;
+}
+constexpr float kGaussScale = -0.72134752044448170368f;  // -log2(e) / 2
+__device__ __forceinline__ float gauss_weight(float log2_o, float v) {
+    return ex2_approx(__fmaf_rn(v, kGaussScale, log2_o));
 }
 __device__ __forceinline__ float gauss_alpha(float log2_o, float v) { return fminf(0.99f, gauss_weight(log2_o, v)); }
 

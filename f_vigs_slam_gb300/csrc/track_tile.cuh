@@ -142,7 +142,7 @@ __device__ __forceinline__ void load_ref_record(const TrackArgs& a, uint32_t g, 
     r2 = make_float4(ph.y, a.ref_col[3 * (size_t)g], a.ref_col[3 * (size_t)g + 1], a.ref_col[3 * (size_t)g + 2]);
 }
 
-// Rejection of a Gaussian by a warp's 8 x ROWS pixel block, once per staged
+// Rejection of a Gaussian by a warp's COLS x ROWS pixel block, once per staged
 // Gaussian.  A pixel skips a Gaussian when v > vreject (alpha < 1/255, both
 // passes) or, in the forward pass only, when v <= 0.  If the extremes of v
 // over the block prove one of these for every pixel -- kRejectAlpha: min v >
@@ -163,12 +163,12 @@ __device__ __forceinline__ void load_ref_record(const TrackArgs& a, uint32_t g, 
 // minimum where it is convex, else a maximum).  The stationary points come
 // from rcp.approx: one ulp off changes v by 1e-14 of its terms.
 constexpr uint32_t kRejectAlpha = 1u, kRejectSign = 2u;
-template <int ROWS = 4>
+template <int ROWS = 4, int COLS = 8>
 __device__ __forceinline__ uint32_t block_reject(float u, float v, float ca, float cb, float cc, float vrej, float x0,
                                                  float y0) {
     if (vrej == -INFINITY) return kRejectAlpha;  // zero opacity: alpha is 0 everywhere
     if (!(isfinite(u) && isfinite(v) && isfinite(ca) && isfinite(cb) && isfinite(cc) && isfinite(vrej))) return 0u;
-    const float dxlo = u - (x0 + 7.0f), dxhi = u - x0;
+    const float dxlo = u - (x0 + (float)(COLS - 1)), dxhi = u - x0;
     const float dylo = v - (y0 + (float)(ROWS - 1)), dyhi = v - y0;
     const float mx = fmaxf(fabsf(dxlo), fabsf(dxhi)), my = fmaxf(fabsf(dylo), fabsf(dyhi));
     const float margin = 1e-5f * (fabsf(ca) * mx * mx + 2.0f * fabsf(cb) * mx * my + fabsf(cc) * my * my) + 1e-3f;

@@ -287,3 +287,33 @@ def test_maintenance_on_empty_map_and_errors(fvgs_lib):
         assert s.remove_outliers(pose, K) == 0
         assert s.prune() == 0
         assert s.visibility(pose, K, W, H)[1] == 0
+
+
+@pytest.mark.parametrize("quirks", [0x4 | 0x8, 0x0], ids=["ref", "intended"])
+@pytest.mark.parametrize("n", [1, 32, 33, 129, 400])
+@pytest.mark.parametrize("size", [(16, 16), (21, 13), (32, 5)])
+def test_outlier_scores_list_and_tile_edges(oracle, fvgs_lib, size, n, quirks):
+    """Lists around a warp's 32 entries and the four warps' 128, tiles cut by
+    the image's edges, and entries whose depth plane passes behind the camera.
+    An exponent's terms stay below 768 (conic 3, 16 pixels) in four FP32
+    operations: 1e-4 of a weight."""
+    W, H = size
+    K = (30.0, 30.0, (W - 1) / 2.0, (H - 1) / 2.0)
+    rng = np.random.default_rng(100 * n + W)
+    scene = S.cam_box(n, seed=n)
+    scene.positions[:, :2] = rng.uniform(-0.3, 0.3, (n, 2)) * scene.positions[:, 2:]
+    scene.scales[:] = rng.uniform(0.1, 0.6, (n, 3))
+    P = oracle.default_params(quirks)
+    pose = (np.zeros(3, np.float32), S.IDENTITY_Q)
+    rgb, obs, gx, gy = _outlier_frame(oracle, scene, pose, K, W, H, P)
+    b = oracle.prepare(scene, pose, K, W, H, P)
+    ta, op = oracle.outlier_scores(b, obs, W, H, P)
+    with _session(fvgs_lib, scene, W, H, quirks) as s:
+        s.set_frame(0, rgb, obs, gx, gy)
+        s.remove_outliers(pose, K, level=0, threshold=0.6, remove=False)
+        _, gta, gop = s.download_marks(n, scores=True)
+    for g, o in ((gta, ta), (gop, op)):
+        with np.errstate(over="ignore", invalid="ignore"):
+            g, o = g.astype(np.float64), o.astype(np.float32).astype(np.float64)
+            near = (g == o) | (np.abs(g - o) <= 1e-4 * np.maximum(1.0, np.abs(o)))
+        assert near.mean() >= 0.99, (near.mean(), g[~near][:4], o[~near][:4])
