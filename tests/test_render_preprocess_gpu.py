@@ -139,3 +139,34 @@ def test_session_stream_follows_set_stream(fvgs_lib):
         assert s.stream() == (st.cuda_stream, 0)
         s.set_stream(None)
         assert s.stream() == (own, 0)
+
+
+@pytest.mark.parametrize("signed", [False, True])
+@pytest.mark.parametrize("n", [1, 32, 33, 200])
+@pytest.mark.parametrize("size", [(16, 16), (21, 13), (9, 5)])
+def test_render_view_list_and_block_edges(oracle, fvgs_lib, size, n, signed):
+    """Lists around a warp's 32 entries and 8 x 8 pixel blocks partly or wholly
+    outside the image, with and without negative opacities; the tolerances of
+    the whole image."""
+    fv = fvgs_lib
+    W, H = size
+    K = (30.0, 30.0, (W - 1) / 2.0, (H - 1) / 2.0)
+    rng = np.random.default_rng(100 * n + W)
+    scene = S.cam_box(n, seed=n)
+    scene.positions[:, :2] = rng.uniform(-0.3, 0.3, (n, 2)) * scene.positions[:, 2:]
+    scene.scales[:] = rng.uniform(0.1, 0.4, (n, 3))
+    if signed:
+        scene.opacities[rng.random(n) < 0.1] *= -0.2
+    P = oracle.default_params(0x8)
+    pose = (np.zeros(3, np.float32), S.IDENTITY_Q)
+    b = oracle.prepare(scene, pose, K, W, H, P)
+    col_o, dep_o = oracle.render_view(scene, b, W, H, P)
+    with fv.Session(n, W, H, fv.default_params(0x8)) as s:
+        s.upload(scene)
+        col, dep, _ = s.render_view(pose, K, W, H, rgb8=True)
+    assert rel_err(col, col_o) <= 1e-5
+    crossed_o, crossed = dep_o < 1e9, dep < 1e9
+    assert (crossed != crossed_o).mean() <= 0.01
+    both = crossed & crossed_o
+    d = np.abs(dep[both] - dep_o[both]) / np.maximum(np.abs(dep_o[both]), 1.0)
+    assert both.sum() == 0 or np.quantile(d, 0.99) <= 1e-5
