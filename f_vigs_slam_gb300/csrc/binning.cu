@@ -173,9 +173,10 @@ __device__ __forceinline__ void project_one(const ProjectArgs& a, int i, float4 
         const bool swap = (a.quirks & FVGS_Q_INVSIGMA_SWAP) != 0;
         const float4 r0 = make_float4(u, v, z, co.w);
         const float4 r1 = make_float4(ixx, swap ? iyy : ixy, swap ? ixy : iyy, phx);
-        a.rec0[i] = r0;
-        a.rec1[i] = r1;
-        a.rec2[i] = make_float4(phy, co.x, co.y, co.z);
+        const float lo2 = log2_opacity(r0.w);
+        float4* rec = a.rec + kRecQuads * (size_t)i;
+        store_pair(rec, r0, r1);
+        store_pair(rec + 2, make_float4(phy, co.x, co.y, co.z), make_float4(lo2, reject_bound(r0.w, lo2), 0.f, 0.f));
         a.bins[i].p = make_float4(u, v, z, phx);
         if constexpr (DERIV) pose_derivs(K.fx, K.fy, swap, r0, r1, geo0, geo1, a.deriv + 8 * (size_t)i);
     }

@@ -143,7 +143,7 @@ struct fvgs_session {
     std::vector<void*> allocations;
 
     float4 *pos = nullptr, *scale = nullptr, *rot = nullptr, *col = nullptr;
-    float4 *rec0 = nullptr, *rec1 = nullptr, *rec2 = nullptr;
+    float4* rec = nullptr;  // kRecQuads per Gaussian
     // pose derivatives of the analytic pose Jacobian (sessions whose quirks
     // clear FVGS_Q_POSE_JAC_APPROX), 8 vectors per Gaussian
     float4* deriv = nullptr;
@@ -659,9 +659,7 @@ int enqueue_bin(fvgs_session* s, const fvgs_intrinsics* K, int W, int H, int tw,
     pa.nty = nty;
     pa.radius_sigma = P.radius_sigma;
     pa.quirks = P.quirks;
-    pa.rec0 = s->rec0;
-    pa.rec1 = s->rec1;
-    pa.rec2 = s->rec2;
+    pa.rec = s->rec;
     pa.bins = s->bins;
     pa.counts = s->counts;
     pa.deriv = track ? s->deriv : nullptr;
@@ -786,9 +784,7 @@ TrackArgs make_track_args(fvgs_session* s, const fvgs_intrinsics* K, const Frame
                           bool images) {
     const fvgs_params& P = s->params;
     TrackArgs ta{};
-    ta.rec0 = s->rec0;
-    ta.rec1 = s->rec1;
-    ta.rec2 = s->rec2;
+    ta.rec = s->rec;
     ta.ranges = s->ranges;
     ta.indices = s->vals;
     ta.n_list = (uint32_t)std::min<uint64_t>(s->cap_inst, 0xffffffffu);
@@ -902,9 +898,7 @@ int enqueue_map(fvgs_session* s, const fvgs_intrinsics* K, const FrameLevel& f, 
     const bool cap = (P.quirks & FVGS_Q_MAP_CAP256) != 0;
     const int ntx = (f.W + P.tile_w - 1) / P.tile_w, nty = (f.H + P.tile_h - 1) / P.tile_h;
     MapArgs ma{};
-    ma.rec0 = s->rec0;
-    ma.rec1 = s->rec1;
-    ma.rec2 = s->rec2;
+    ma.rec = s->rec;
     ma.ranges = s->ranges;
     ma.indices = s->vals;
     ma.n_list = (uint32_t)std::min<uint64_t>(s->cap_inst, 0xffffffffu);
@@ -1067,9 +1061,7 @@ int fvgs_session_create(const fvgs_params* params, int device, uint32_t capacity
     FV_A(s->scale, N);
     FV_A(s->rot, N);
     FV_A(s->col, N);
-    FV_A(s->rec0, N);
-    FV_A(s->rec1, N);
-    FV_A(s->rec2, N);
+    FV_A(s->rec, kRecQuads * N);
     if (!(P.quirks & FVGS_Q_POSE_JAC_APPROX)) {
         FV_A(s->deriv, 8 * N);
     }
@@ -1252,11 +1244,11 @@ int fvgs_upload_gaussians(fvgs_session* s, const float* positions, const float* 
     ctx_drop_history(s);
     FV_CK(cand_drop(s));
     if (n == 0) return FVGS_OK;
-    // Stage through rec planes (free until the next binning) so host arrays of
+    // Stage through the records (free until the next binning) so host arrays of
     // the reference's float3 layout become 16-byte vectors on the device.
-    float* tmp = reinterpret_cast<float*>(s->rec0);  // 4N floats
-    float* tmp2 = reinterpret_cast<float*>(s->rec1);
-    float* tmp3 = reinterpret_cast<float*>(s->rec2);
+    float* tmp = reinterpret_cast<float*>(s->rec);  // 4N floats
+    float* tmp2 = reinterpret_cast<float*>(s->rec + s->cap_g);
+    float* tmp3 = reinterpret_cast<float*>(s->rec + 2 * (size_t)s->cap_g);
     float* tmp4 = reinterpret_cast<float*>(s->bins);       // 8N floats
     float* tmp5 = reinterpret_cast<float*>(s->offsets);
     FV_CK(cudaMemcpyAsync(tmp, positions, sizeof(float) * 3 * n, cudaMemcpyDefault, s->stream));
@@ -1280,9 +1272,9 @@ int fvgs_download_gaussians(fvgs_session* s, float* positions, float* scales, fl
         return FVGS_E_INVALID;
     FV_CK(cudaSetDevice(s->device));
     if (n == 0) return FVGS_OK;
-    float* tmp = reinterpret_cast<float*>(s->rec0);
-    float* tmp2 = reinterpret_cast<float*>(s->rec1);
-    float* tmp3 = reinterpret_cast<float*>(s->rec2);
+    float* tmp = reinterpret_cast<float*>(s->rec);
+    float* tmp2 = reinterpret_cast<float*>(s->rec + s->cap_g);
+    float* tmp3 = reinterpret_cast<float*>(s->rec + 2 * (size_t)s->cap_g);
     float* tmp4 = reinterpret_cast<float*>(s->bins);       // 8N floats
     float* tmp5 = reinterpret_cast<float*>(s->offsets);
     download_unpack_kernel<<<(n + 255) / 256, 256, 0, s->stream>>>(s->pos, s->scale, s->rot, s->col, n, tmp, tmp2,
@@ -1458,10 +1450,8 @@ int fvgs_download_projection(fvgs_session* s, float* uv, float* cov2d, float* in
     if ((cov2d || inv2d || visible) && !s->dbg_proj_valid) return FVGS_E_STATE;
     FV_CK(cudaSetDevice(s->device));
     const size_t n = s->n_g;
-    std::vector<float4> r0(n), r1(n), r2(n);
-    FV_CK(cudaMemcpyAsync(r0.data(), s->rec0, sizeof(float4) * n, cudaMemcpyDeviceToHost, s->stream));
-    FV_CK(cudaMemcpyAsync(r1.data(), s->rec1, sizeof(float4) * n, cudaMemcpyDeviceToHost, s->stream));
-    FV_CK(cudaMemcpyAsync(r2.data(), s->rec2, sizeof(float4) * n, cudaMemcpyDeviceToHost, s->stream));
+    std::vector<float4> rec(kRecQuads * n);
+    FV_CK(cudaMemcpyAsync(rec.data(), s->rec, sizeof(float4) * rec.size(), cudaMemcpyDeviceToHost, s->stream));
     if (cov2d) FV_CK(cudaMemcpyAsync(cov2d, s->dbg_cov, sizeof(float) * 3 * n, cudaMemcpyDefault, s->stream));
     if (inv2d) FV_CK(cudaMemcpyAsync(inv2d, s->dbg_inv, sizeof(float) * 3 * n, cudaMemcpyDefault, s->stream));
     if (visible) FV_CK(cudaMemcpyAsync(visible, s->dbg_vis, n, cudaMemcpyDefault, s->stream));
@@ -1472,15 +1462,16 @@ int fvgs_download_projection(fvgs_session* s, float* uv, float* cov2d, float* in
     for (size_t i = 0; i < n; ++i) {
         // Gaussians without instances keep no record on the device; the
         // reference's buffers hold zeros for them
-        if (cnt[i] == 0) r0[i] = r1[i] = r2[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (cnt[i] == 0) std::fill_n(rec.begin() + kRecQuads * i, kRecQuads, make_float4(0.f, 0.f, 0.f, 0.f));
+        const float4* r = rec.data() + kRecQuads * i;
         if (uv) {
-            uv[2 * i] = r0[i].x;
-            uv[2 * i + 1] = r0[i].y;
+            uv[2 * i] = r[0].x;
+            uv[2 * i + 1] = r[0].y;
         }
-        if (depth) depth[i] = r0[i].z;
+        if (depth) depth[i] = r[0].z;
         if (phat) {
-            phat[2 * i] = r1[i].w;
-            phat[2 * i + 1] = r2[i].x;
+            phat[2 * i] = r[1].w;
+            phat[2 * i + 1] = r[2].x;
         }
     }
     return FVGS_OK;
@@ -2731,9 +2722,7 @@ int fvgs_render_view(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsi
         FV_TRY(set_pose(s, pose));
         FV_TRY(enqueue_bin(s, K, width, height, s->params.tile_w, s->params.tile_h));
         RenderArgs ra{};
-        ra.rec0 = s->rec0;
-        ra.rec1 = s->rec1;
-        ra.rec2 = s->rec2;
+        ra.rec = s->rec;
         ra.ranges = s->ranges;
         ra.indices = s->vals;
         ra.n_list = (uint32_t)std::min<uint64_t>(s->cap_inst, 0xffffffffu);
@@ -2855,8 +2844,7 @@ int visibility_pass(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsic
         FV_TRY(enqueue_bin(s, K, W, H, s->params.tile_w, s->params.tile_h));
         FV_CK(cudaMemsetAsync(vis, 0, s->n_g, s->stream));
         VisArgs va{};
-        va.rec0 = s->rec0;
-        va.rec1 = s->rec1;
+        va.rec = s->rec;
         va.ranges = s->ranges;
         va.indices = s->vals;
         va.n_list = (uint32_t)std::min<uint64_t>(s->cap_inst, 0xffffffffu);
@@ -3015,9 +3003,7 @@ int fvgs_remove_outliers(fvgs_session* s, const fvgs_pose* pose, const fvgs_intr
         FV_CK(cudaMemsetAsync(s->mk_total_alpha, 0, sizeof(float) * s->n_g, s->stream));
         FV_CK(cudaMemsetAsync(s->mk_outlier_prob, 0, sizeof(float) * s->n_g, s->stream));
         OutlierArgs oa{};
-        oa.rec0 = s->rec0;
-        oa.rec1 = s->rec1;
-        oa.rec2 = s->rec2;
+        oa.rec = s->rec;
         oa.ranges = s->ranges;
         oa.indices = s->vals;
         oa.n_list = (uint32_t)std::min<uint64_t>(s->cap_inst, 0xffffffffu);
@@ -3183,9 +3169,7 @@ int fvgs_densify(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics* 
         FV_TRY(set_pose(s, pose));
         FV_TRY(enqueue_bin(s, K, W, H, s->params.tile_w, s->params.tile_h));
         DensityArgs da{};
-        da.rec0 = s->rec0;
-        da.rec1 = s->rec1;
-        da.rec2 = s->rec2;
+        da.rec = s->rec;
         da.ranges = s->ranges;
         da.indices = s->vals;
         da.n_list = (uint32_t)std::min<uint64_t>(s->cap_inst, 0xffffffffu);

@@ -7,10 +7,13 @@
 //     g_scale[N] float4 (sx, sy, sz, 0)
 //     g_rot[N]   float4 (x, y, z, w)      raw quaternion as the reference reads it
 //     g_col[N]   float4 (r, g, b, opacity)
-//   Blending record, 48 B per Gaussian (three float4 planes):
-//     rec0 = (u, v, z, opacity)
-//     rec1 = (c.x, c.y, c.z, phat.x)      c = inverse 2D covariance in the order
-//     rec2 = (phat.y, r, g, b)             the blending kernels consume it
+//   Blending record, 64 B per Gaussian (four float4, so that a gather takes two
+//   whole sectors; three planes of float4 cost three half sectors and a line
+//   each):
+//     (u, v, z, opacity)
+//     (c.x, c.y, c.z, phat.x)              c = inverse 2D covariance in the order
+//     (phat.y, r, g, b)                    the blending kernels consume it
+//     (log2(opacity), reject_bound, 0, 0)
 //   Reduced-precision attributes (precision form; the float4 planes stay the
 //   master copy that mapping updates):
 //     g_sr[N]    uint4 scale bf16 x3, rotation bf16 x4 (raw order), 2 B spare
@@ -31,6 +34,14 @@
 namespace fvgs {
 
 constexpr uint32_t kFullMask = 0xffffffffu;
+constexpr int kRecQuads = 4;  // float4 of a blending record
+
+// Two float4 to a 32-byte boundary in one store (a whole sector).
+__device__ __forceinline__ void store_pair(float4* p, const float4& a, const float4& b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
 
 // Device-side status word bits (session->status[0]); host reads after a step.
 constexpr uint32_t kErrOverflow = 1u << 0;  // instance capacity exceeded

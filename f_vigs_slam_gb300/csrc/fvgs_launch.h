@@ -77,9 +77,7 @@ struct ProjectArgs {
     float inv_tw, inv_th;
     float radius_sigma;
     uint32_t quirks;
-    float4* rec0;
-    float4* rec1;
-    float4* rec2;
+    float4* rec;
     BinRec* bins;
     uint32_t* counts;
     int* tile_diff;    // optional: binning scratch (tile_diff_words): count grid, entering grid, counters
@@ -208,9 +206,7 @@ cudaError_t launch_radix_sort(uint64_t* keys, uint32_t* vals, const DevStatus* s
 
 // ---- tracking (track.cu) ----
 struct TrackArgs {
-    const float4* rec0;
-    const float4* rec1;
-    const float4* rec2;
+    const float4* rec;
     const uint2* ranges;
     const uint32_t* indices;
     // list entries at or beyond n_list and indices at or above n_gauss are
@@ -325,9 +321,7 @@ cudaError_t track_batch_configure_device();
 
 // ---- render form (render.cu) ----
 struct RenderArgs {
-    const float4* rec0;
-    const float4* rec1;
-    const float4* rec2;
+    const float4* rec;
     const uint2* ranges;
     const uint32_t* indices;
     uint32_t n_list, n_gauss;  // as TrackArgs
@@ -351,9 +345,7 @@ cudaError_t launch_prep_level(const uint8_t* prev, const float* prev_depth, int 
 
 // ---- mapping (map.cu) ----
 struct MapArgs {
-    const float4* rec0;
-    const float4* rec1;
-    const float4* rec2;
+    const float4* rec;
     const uint2* ranges;
     const uint32_t* indices;
     uint32_t n_list;   // as TrackArgs
@@ -399,8 +391,7 @@ cudaError_t launch_pack_reduced(const float4* scale, const float4* rot, const fl
 
 // ---- map maintenance (maintenance.cu) ----
 struct VisArgs {
-    const float4* rec0;
-    const float4* rec1;
+    const float4* rec;
     const uint2* ranges;
     const uint32_t* indices;
     uint32_t n_list, n_gauss;  // as TrackArgs
@@ -409,9 +400,7 @@ struct VisArgs {
     uint8_t* vis;  // [n_gauss], set to 1 where visible (cleared by the caller)
 };
 struct OutlierArgs {
-    const float4* rec0;
-    const float4* rec1;
-    const float4* rec2;
+    const float4* rec;
     const uint2* ranges;
     const uint32_t* indices;
     uint32_t n_list, n_gauss;
@@ -472,9 +461,7 @@ struct SeedArgs {
     float4* adam;  // emit: zero the optimiser state of each seed (null: leave it)
 };
 struct DensityArgs {
-    const float4* rec0;
-    const float4* rec1;
-    const float4* rec2;
+    const float4* rec;
     const uint2* ranges;
     const uint32_t* indices;
     uint32_t n_list, n_gauss;

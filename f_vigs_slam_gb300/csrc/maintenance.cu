@@ -9,8 +9,8 @@
 // remove the marked Gaussians with thrust::sort_by_key on the 0 / 0xff states
 // (survivors first, in order) and shrink the Gaussian count.
 //
-// Every blending kernel here reads the packed records of the binning (rec0 =
-// u, v, z, opacity; rec1 = c.x, c.y, c.z, phat.x; rec2 = phat.y, rgb), where
+// Every blending kernel here reads the packed records of the binning (u,
+// v, z, opacity; c.x, c.y, c.z, phat.x; phat.y, rgb; ...), where
 // c is the inverse 2D covariance in the order the reference's tracking
 // kernels consume it (c.y as the xy term, c.z as the yy term).  The
 // reference's visibility and outlier kernels read the stored inverse the same
@@ -72,8 +72,8 @@ __global__ void __launch_bounds__(kMPix) visibility_kernel(VisArgs a) {
             g = a.indices[range.x + li];
             float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
             if (g < a.n_gauss) {
-                r0 = a.rec0[g];
-                r1 = a.rec1[g];
+                r0 = a.rec[kRecQuads * (size_t)g];
+                r1 = a.rec[kRecQuads * (size_t)g + 1];
             }
             constexpr float kNegHalfLog2e = -0.72134752044448170368f;
             sA[tid] = make_float4(r0.x, r0.y, log2_opacity(r0.w), kNegHalfLog2e * r1.x);
@@ -216,14 +216,15 @@ __global__ void __launch_bounds__(32 * kOutWarps) outliers_kernel(OutlierArgs a)
             OutlierEntry e;
             bool keep = false;
             if (g < a.n_gauss) {
-                const float4 r0 = a.rec0[g], r1 = a.rec1[g];
+                const float4* rec = a.rec + kRecQuads * (size_t)g;
+                const float4 r0 = rec[0], r1 = rec[1], r3 = rec[3];
                 e.u = r0.x, e.v = r0.y, e.z = r0.z;
-                e.lo2 = log2_opacity(r0.w);  // alpha = o exp(-q/2) = 2^(log2 o - q log2(e) / 2)
+                e.lo2 = r3.x;  // log2 o; alpha = o exp(-q/2) = 2^(log2 o - q log2(e) / 2)
                 e.ca = r1.x, e.cb = r1.y, e.cc = r1.z, e.phx = r1.w;
-                e.phy = a.rec2[g].x;
+                e.phy = rec[2].x;
                 e.g = g;
                 // a finite bound also for opacity 0, so that non-finite records are kept
-                const float vrej = fmaxf(reject_bound(r0.w, e.lo2), -FLT_MAX);
+                const float vrej = fmaxf(r3.y, -FLT_MAX);
                 keep = !(block_reject<16, 16>(e.u, e.v, e.ca, e.cb, e.cc, vrej, (float)x0, (float)y0) & kRejectAlpha);
             }
             const uint32_t bal = __ballot_sync(kFullMask, keep);

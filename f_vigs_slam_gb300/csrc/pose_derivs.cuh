@@ -64,14 +64,14 @@ __device__ __forceinline__ void pose_derivs(float fx, float fy, bool swap, const
         db[k] = swap ? dq11 : dq01;
         dc[k] = swap ? dq01 : dq11;
     }
-    out[0] = make_float4(du[0], du[1], dv[0], dv[1]);
-    out[1] = make_float4(da[0], da[1], db[0], db[1]);
-    out[2] = make_float4(dc[0], dc[1], du[2], du[3]);
-    out[3] = make_float4(dv[2], dv[3], da[2], da[3]);
-    out[4] = make_float4(db[2], db[3], dc[2], dc[3]);
-    out[5] = make_float4(du[4], du[5], dv[4], dv[5]);
-    out[6] = make_float4(da[4], da[5], db[4], db[5]);
-    out[7] = make_float4(dc[4], dc[5], x, y);
+    store_pair(out, make_float4(du[0], du[1], dv[0], dv[1]),
+               make_float4(da[0], da[1], db[0], db[1]));
+    store_pair(out + 2, make_float4(dc[0], dc[1], du[2], du[3]),
+               make_float4(dv[2], dv[3], da[2], da[3]));
+    store_pair(out + 4, make_float4(db[2], db[3], dc[2], dc[3]),
+               make_float4(du[4], du[5], dv[4], dv[5]));
+    store_pair(out + 6, make_float4(da[4], da[5], db[4], db[5]),
+               make_float4(dc[4], dc[5], x, y));
 }
 
 }  // namespace fvgs

@@ -30,7 +30,7 @@ struct ViewStage {
     float4 C[kRound];     // r, r, g, g
     float4 D[kRound];     // b, b, c'xx, c'xx
     float S[kRound];      // sign of the opacity (read only by rounds with an odd record)
-    float4 R[3][kRound];  // the next round's records, in flight
+    RecordStage R;        // the next round's records, in flight
 };
 
 // w = o exp(-q/2) as 2^t with t = log2|o| + c'xx dx^2 + 2 c'xy dx dy +
@@ -133,14 +133,7 @@ __global__ void __launch_bounds__(64) render_view_kernel(RenderArgs a) {
     };
 
     // the records of the next round travel while this one's are blended
-    auto fetch = [&](uint32_t g) {
-        if (g < a.n_gauss) {
-            cp_async16(&ws.R[0][lane], a.rec0 + g);
-            cp_async16(&ws.R[1][lane], a.rec1 + g);
-            cp_async16(&ws.R[2][lane], a.rec2 + g);
-        }
-        cp_async_commit();
-    };
+    auto fetch = [&](uint32_t g) { fetch_records(ws.R, a.rec, g, a.n_gauss); };
     uint32_t g = lane < n ? a.indices[range.x + lane] : 0xffffffffu;
     if (!__all_sync(kFullMask, done)) {
         fetch(g);
@@ -149,10 +142,11 @@ __global__ void __launch_bounds__(64) render_view_kernel(RenderArgs a) {
             const uint32_t g_next = li + kRound < n ? a.indices[range.x + li + kRound] : 0xffffffffu;
             float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
             cp_async_wait<0>();
+            __syncwarp();  // four lanes brought each record
             if (g < a.n_gauss) {
-                r0 = ws.R[0][lane];
-                r1 = ws.R[1][lane];
-                r2 = ws.R[2][lane];
+                r0 = record_quad(ws.R, lane, 0);
+                r1 = record_quad(ws.R, lane, 1);
+                r2 = record_quad(ws.R, lane, 2);
             }
             // the packed record holds the inverse in the tracking kernels'
             // consumed order; undo the swap for the true layout

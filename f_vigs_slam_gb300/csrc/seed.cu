@@ -272,9 +272,9 @@ __global__ void __launch_bounds__(256) density_mask_kernel(DensityArgs a) {
             const uint32_t g = a.indices[range.x + li];
             float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
             if (g < a.n_gauss) {
-                r0 = a.rec0[g];
-                r1 = a.rec1[g];
-                r2 = a.rec2[g];
+                r0 = a.rec[kRecQuads * (size_t)g];
+                r1 = a.rec[kRecQuads * (size_t)g + 1];
+                r2 = a.rec[kRecQuads * (size_t)g + 2];
             }
             sA[tid] = make_float4(r0.x, r0.y, r0.w, r1.x);
             sB[tid] = make_float4(r1.y, r1.z, r0.z, r1.w);
