@@ -933,9 +933,16 @@ cudaError_t launch_copy_lists(const uint2* ranges, int T, const uint32_t* src, u
 
 cudaError_t launch_project_count(const ProjectArgs& a, int max_ctas, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
-    const int need = (a.n + kProjChunk - 1) / kProjChunk;
-    return launch_chained(a.deriv ? project_count_kernel<true> : project_count_kernel<false>, dim3(max_ctas > 0 && max_ctas < need ? max_ctas : need), dim3(256), 0,
-                          s, a);
+    // CTAs for one Gaussian a thread, up to the cap; a chunk of two a thread is
+    // for the passes of a capped grid.  With CTAs for whole chunks a small
+    // map left SMs idle and its threads two projections in series (50 k
+    // Gaussians, VGA: 15.7 us against 13.8; 2 k, 160x120: 13.1 against 11.0).  Wider CTAs
+    // flush fewer copies of the difference grids but end later: 512 threads
+    // gain 1.4 us at 1 M Gaussians HD and lose as much on longer lists.
+    const int need = (a.n + kProjThreads - 1) / kProjThreads;
+    const int grid = max_ctas > 0 && max_ctas < need ? max_ctas : need;
+    return launch_chained(a.deriv ? project_count_kernel<true> : project_count_kernel<false>, dim3(grid),
+                          dim3(kProjThreads), 0, s, a);
 }
 
 size_t scan_partials_size(int n) { return (size_t)((n + kScanBlock - 1) / kScanBlock); }
