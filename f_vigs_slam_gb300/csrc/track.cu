@@ -301,6 +301,18 @@ __device__ __forceinline__ void track_reduce_body(const float* __restrict__ tile
         for (int ww = 0; ww < 8; ++ww) c += s_w[ww][lane];
         s_part[lane] = c;
     }
+    // warp 1, while the cluster meets: lane i < 3 the row i of R, the rotation
+    // of the pose the Jacobians were taken at
+    double r0 = 0.0, r1 = 0.0, r2 = 0.0;
+    if (DO_GN && rank == 0 && w == 1) {
+        const double qx = pq[0], qy = pq[1], qz = pq[2], qw = pq[3];
+        const double R[3][3] = {
+            {1.0 - 2.0 * (qy * qy + qz * qz), 2.0 * (qx * qy - qw * qz), 2.0 * (qx * qz + qw * qy)},
+            {2.0 * (qx * qy + qw * qz), 1.0 - 2.0 * (qx * qx + qz * qz), 2.0 * (qy * qz - qw * qx)},
+            {2.0 * (qx * qz - qw * qy), 2.0 * (qy * qz + qw * qx), 1.0 - 2.0 * (qx * qx + qy * qy)}};
+        auto row = [&](int j) { return lane == 0 ? R[0][j] : (lane == 1 ? R[1][j] : R[2][j]); };
+        r0 = row(0), r1 = row(1), r2 = row(2);
+    }
     cluster.sync();  // every CTA's column sums are visible cluster-wide
     if (rank == 0 && w == 0 && lane < FVGS_POSEDATA_FLOATS) {
         double c = 0.0;
@@ -423,29 +435,25 @@ __device__ __forceinline__ void track_reduce_body(const float* __restrict__ tile
     double x[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) x[k] = shfl_d(xv, k);
-    if (lane != 0) return;
-    // delta = (R x_t, x_r), R of the pose the Jacobians were taken at
-    const double qx = pq[0], qy = pq[1], qz = pq[2], qw = pq[3];
-    const double R[3][3] = {
-        {1.0 - 2.0 * (qy * qy + qz * qz), 2.0 * (qx * qy - qw * qz), 2.0 * (qx * qz + qw * qy)},
-        {2.0 * (qx * qy + qw * qz), 1.0 - 2.0 * (qx * qx + qz * qz), 2.0 * (qy * qz - qw * qx)},
-        {2.0 * (qx * qz - qw * qy), 2.0 * (qy * qz + qw * qx), 1.0 - 2.0 * (qx * qx + qy * qy)}};
-    double delta[6];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) delta[i] = R[i][0] * x[0] + R[i][1] * x[1] + R[i][2] * x[2];
-#pragma unroll
-    for (int i = 3; i < 6; ++i) delta[i] = x[i];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        ptd[k] += delta[k];
-        pose->td[k] = ptd[k];
+    // A component a lane, which takes 27 FP64 instructions in series instead of
+    // the 120 of one thread.  delta = (R x_t, x_r): lane k < 6 its component k.
+    const double delta = lane < 3 ? r0 * x[0] + r1 * x[1] + r2 * x[2] : xv;
+    if (step_out && lane < 6) step_out[lane] = delta;
+    if (lane < 3) {
+        const double td = (lane == 0 ? ptd[0] : (lane == 1 ? ptd[1] : ptd[2])) + delta;
+        pose->td[lane] = td;
+        pose->t[lane] = (float)td;
     }
     const double ax = pqd[0], ay = pqd[1], az = pqd[2], aw = pqd[3];
-    const double bx = 0.5 * delta[3], by = 0.5 * delta[4], bz = 0.5 * delta[5];
-    double nx = aw * bx + ax + (ay * bz - az * by);
-    double ny = aw * by + ay + (az * bx - ax * bz);
-    double nz = aw * bz + az + (ax * by - ay * bx);
-    double nw = aw - (ax * bx + ay * by + az * bz);
+    const double bx = 0.5 * x[3], by = 0.5 * x[4], bz = 0.5 * x[5];
+    // lane i < 3: the vector part's component i, aw b + a + a x b; lane 3: the scalar
+    auto pick3 = [&](int i, double u, double v, double t) { return i == 0 ? u : (i == 1 ? v : t); };
+    const int c0 = lane < 3 ? lane : 0, c1 = c0 == 2 ? 0 : c0 + 1, c2 = c1 == 2 ? 0 : c1 + 1;
+    const double a0 = pick3(c0, ax, ay, az), a1 = pick3(c1, ax, ay, az), a2 = pick3(c2, ax, ay, az);
+    const double b0 = pick3(c0, bx, by, bz), b1 = pick3(c1, bx, by, bz), b2 = pick3(c2, bx, by, bz);
+    const double nv = aw * b0 + a0 + (a1 * b2 - a2 * b1);
+    const double nw = aw - (ax * bx + ay * by + az * bz);
+    const double nx = shfl_d(nv, 0), ny = shfl_d(nv, 1), nz = shfl_d(nv, 2);
     // 1 / |n| by the FP32 estimate and two Newton steps r *= (3 - n2 r^2) / 2
     // (about 2^-22, 2^-44, then rounding): the quaternion is within O(|delta|^2)
     // of unit length, and FP64 square root and division are long chains here
@@ -453,23 +461,11 @@ __device__ __forceinline__ void track_reduce_body(const float* __restrict__ tile
     double inn = (double)rsqrtf((float)n2);
     inn = inn * fma(-0.5 * n2, inn * inn, 1.5);
     inn = inn * fma(-0.5 * n2, inn * inn, 1.5);
-    nx *= inn;
-    ny *= inn;
-    nz *= inn;
-    nw *= inn;
-    pose->qd[0] = nx;
-    pose->qd[1] = ny;
-    pose->qd[2] = nz;
-    pose->qd[3] = nw;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) pose->t[k] = (float)ptd[k];
-    pose->q[0] = (float)nx;
-    pose->q[1] = (float)ny;
-    pose->q[2] = (float)nz;
-    pose->q[3] = (float)nw;
-    if (step_out)
-#pragma unroll
-        for (int k = 0; k < 6; ++k) step_out[k] = delta[k];
+    const double q = (lane < 3 ? nv : nw) * inn;
+    if (lane < 4) {
+        pose->qd[lane] = q;
+        pose->q[lane] = (float)q;
+    }
 }
 
 template <bool DO_GN>
