@@ -346,18 +346,20 @@ def algorithmic_bytes(cls, n_g, n_vis, n_inst, visited, W, H, n_cand=None):
     if n_cand is None:
         proj = (20 * n_g + 160 * n_vis,
                 "20 B per Gaussian (position, previous count) + per visible Gaussian 48 B of attributes in and "
-                "112 B out (blending 48, binning 32, geometry 32 records)")
+                "112 B out (blending 48, binning 32, geometry 32; stored as 64, 32 and 128)")
     else:
         proj = (24 * n_cand + 160 * n_vis,
                 "candidate list reused: 24 B per listed Gaussian (index, position, previous count) + per visible "
-                "Gaussian 48 B of attributes in and 112 B out (blending 48, binning 32, geometry 32 records)")
+                "Gaussian 48 B of attributes in and 112 B out (blending 48, binning 32, geometry 32; stored as 64, 32 "
+                "and 128)")
     table = {
         "project": proj,
         "sort": (8 * n_inst + 32 * n_vis,
                  "incremental per-tile sort: 4 B in + 4 B out per instance + each visible Gaussian's 32-byte "
                  "binning record"),
         "track": (80 * visited + 16 * P + 108 * T,
-                  "48-byte blending + 32-byte geometry record per instance read (list prefixes the pixels reach), "
+                  "48 bytes of blending record + the 32 bytes of geometry its pose derivatives are made from per "
+                  "instance read (list prefixes the pixels reach; stored as 64 and 128), "
                   "16 B per pixel of observed colour and depth, 108 B per tile out"),
         "gn": (108 * T, "the tile partials"),
         "map_fwd": (48 * visited + 52 * P, "48-byte record per instance read + 16 B in and 36 B out per pixel"),

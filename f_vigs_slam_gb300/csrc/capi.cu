@@ -2737,7 +2737,7 @@ int fvgs_render_view(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsi
         ra.out_rgb8 = rgb8_dev;
         {
             KScope k(s, FVGS_K_RENDER, 1);
-            FV_CK(launch_render_view(ra, s->stream));
+            FV_CK(launch_render_view(ra, s->num_sms, s->stream));
         }
         FV_CK(cudaMemcpyAsync(s->h_st, s->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, s->stream));
         FV_CK(cudaStreamSynchronize(s->stream));
@@ -2800,7 +2800,7 @@ int fvgs_map_step(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics*
         int retry = 0;
         FV_TRY(check_status(s, &retry));
         if (retry) {
-            // the instance buffers grew; checkpoint slots follow capacity
+            // the instance buffers grew
             FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H));
             continue;
         }

@@ -331,7 +331,7 @@ struct RenderArgs {
     float* out_depth;    // P
     uint8_t* out_rgb8;   // optional 3P
 };
-cudaError_t launch_render_view(const RenderArgs& a, cudaStream_t s);
+cudaError_t launch_render_view(const RenderArgs& a, int num_sms, cudaStream_t s);
 
 // ---- frame preprocessing (preprocess.cu) ----
 // Level 0 of a W x H camera frame: depth in metres (float, or uint16 mm), the

@@ -1,4 +1,4 @@
-// map.cu -- mapping step (forward with checkpoints, per-Gaussian backward,
+// map.cu -- mapping step (forward, backward,
 // 2D->3D chain rule and Adam) for sm_103a.
 //
 // Reference: GSSlam::optimizeGaussiansKeyframe (src/GSSlam.cu:1083-1320) with

@@ -18,6 +18,8 @@
 // The reference writes its float3 colour into an 8-bit, 3-channel image (an
 // overrun); here the image is a float RGB buffer, with an optional 8-bit copy
 // (round(255 c), saturated).
+#include <type_traits>
+
 #include "track_tile.cuh"
 
 namespace fvgs {
@@ -200,9 +202,107 @@ __global__ void __launch_bounds__(64) render_view_kernel(RenderArgs a) {
     }
 }
 
-cudaError_t launch_render_view(const RenderArgs& a, cudaStream_t s) {
+// The form for small images: a CTA per tile, a pixel a lane, 256 entries staged
+// by the whole CTA.  It has twice the warps a tile, and its long lists (few
+// tiles: each holds much of the map) are staged eight times as deep.
+constexpr int kRPix = 256;  // 16 x 16 pixels per tile
+__global__ void __launch_bounds__(kRPix) render_view_tile_kernel(RenderArgs a) {
+    pdl_begin();
+    __shared__ float4 sA[kRPix];  // u, v, log2|opacity|, z
+    __shared__ float4 sB[kRPix];  // c'xx, 2 c'xy, c'yy, phat.x
+    __shared__ float4 sC[kRPix];  // phat.y, r, g, b
+    __shared__ float sS[kRPix];   // sign of the opacity (read only by batches with a negative one)
+    const int tile = blockIdx.x;
+    const int tx = tile % a.ntx, ty = tile / a.ntx;
+    const int tid = threadIdx.x;
+    const int x = tx * 16 + (tid & 15), y = ty * 16 + (tid >> 4);
+    const bool inside = x < a.W && y < a.H;
+    uint2 range = a.ranges[tile];
+    range.y = min(range.y, a.n_list);
+    const int n = range.y > range.x ? (int)(range.y - range.x) : 0;
+    const bool swap = (a.quirks & FVGS_Q_INVSIGMA_SWAP) != 0;
+    const float px = (float)x, py = (float)y;
+    float cr = 0.f, cg = 0.f, cb = 0.f, T = 1.f, depth = 1e10f;
+    bool has_depth = false, done = !inside;
+
+    // one pair; NEG: the weight takes the sign of the Gaussian's opacity
+    auto blend = [&](int j, auto neg_tag) {
+        constexpr bool NEG = decltype(neg_tag)::value;
+        const float4 gA = sA[j];
+        const float4 gB = sB[j];
+        const float dx = px - gA.x, dy = py - gA.y;
+        const float t = __fmaf_rn(dx, __fmaf_rn(gB.x, dx, __fmul_rn(gB.y, dy)),
+                                  __fmaf_rn(__fmul_rn(gB.z, dy), dy, gA.z));
+        float w = ex2_approx(t);
+        if (NEG) w *= sS[j];
+        const float Tb = T;
+        const float Tw = Tb * w;
+        const float4 gC = sC[j];
+        cr += Tw * gC.y;
+        cg += Tw * gC.z;
+        cb += Tw * gC.w;
+        T = Tb * (1.0f - w);  // 1 - A of the reference, without the cancellation
+        if (!has_depth && Tb > 0.5f && T <= 0.5f) {
+            depth = gA.w + gB.w * dx + gC.x * dy;
+            has_depth = true;
+        }
+        if (T <= 0.01f) done = true;  // A >= 0.99
+    };
+
+    for (int base = 0; base < n; base += kRPix) {
+        if (__syncthreads_and(done)) break;
+        const int li = base + tid;
+        bool neg = false;
+        if (li < n) {
+            const uint32_t g = a.indices[range.x + li];
+            float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
+            if (g < a.n_gauss) {
+                const float4* rec = a.rec + kRecQuads * (size_t)g;
+                r0 = rec[0];
+                r1 = rec[1];
+                r2 = rec[2];
+            }
+            // the packed record holds the inverse in the tracking kernels'
+            // consumed order; undo the swap for the true layout
+            const float ixy = swap ? r1.z : r1.y, iyy = swap ? r1.y : r1.z;
+            neg = r0.w < 0.f;
+            sA[tid] = make_float4(r0.x, r0.y, log2f(fabsf(r0.w)), r0.z);
+            sB[tid] = make_float4(kGaussScale * r1.x, 2.0f * kGaussScale * ixy, kGaussScale * iyy, r1.w);
+            sC[tid] = r2;
+            sS[tid] = neg ? -1.0f : 1.0f;
+        }
+        const bool any_neg = __syncthreads_or(neg);
+        const int cnt = min(kRPix, n - base);
+        if (!any_neg) {
+            for (int j = 0; j < cnt && !done; ++j) blend(j, std::false_type{});
+        } else {
+            for (int j = 0; j < cnt && !done; ++j) blend(j, std::true_type{});
+        }
+    }
+    if (!inside) return;
+    const size_t p = (size_t)y * a.W + x;
+    a.out_rgb[3 * p] = cr;
+    a.out_rgb[3 * p + 1] = cg;
+    a.out_rgb[3 * p + 2] = cb;
+    a.out_depth[p] = depth;
+    if (a.out_rgb8) {
+        a.out_rgb8[3 * p] = (uint8_t)__float2int_rn(__saturatef(cr) * 255.0f);
+        a.out_rgb8[3 * p + 1] = (uint8_t)__float2int_rn(__saturatef(cg) * 255.0f);
+        a.out_rgb8[3 * p + 2] = (uint8_t)__float2int_rn(__saturatef(cb) * 255.0f);
+    }
+}
+
+// Up to kSmallTiles tiles per SM the warps of two pixels a lane are too few to
+// hide each other's latency.  Kernel, us, that form / the tile's: 107x82 (42
+// tiles) 39 / 29, 160x120 (80) 94 / 66, 240x160 (150) 43 / 31, 398x313 (500) 37 /
+// 37, 500x400 (800) 37 / 39, 640x480 (1200) 41 / 45, 900x600 (2166) 45 / 50,
+// 1280x720 (3600) 64 / 74.
+constexpr int kSmallTiles = 3;
+
+cudaError_t launch_render_view(const RenderArgs& a, int num_sms, cudaStream_t s) {
     const int T = a.ntx * a.nty;
     if (T <= 0) return cudaSuccess;
+    if (T <= kSmallTiles * num_sms) return launch_chained(render_view_tile_kernel, dim3(T), dim3(kRPix), 0, s, a);
     return launch_chained(render_view_kernel, dim3(2 * T), dim3(64), 0, s, a);
 }
 

@@ -37,15 +37,15 @@ typedef struct fvgs_session fvgs_session;
 /* Kernel classes for launch accounting and timing. */
 enum {
     FVGS_K_PROJECT = 0, /* projection + tile count */
-    FVGS_K_SCAN,        /* instance offsets (and mapping bucket offsets) */
+    FVGS_K_SCAN,        /* instance offsets */
     FVGS_K_EMIT,        /* tile-key emission */
-    FVGS_K_SORT,        /* radix sort: histogram + digit passes */
+    FVGS_K_SORT,        /* per-tile sort (or the radix check path) */
     FVGS_K_RANGES,      /* per-tile ranges */
     FVGS_K_TRACK,       /* fused tracking blend + Jacobian */
     FVGS_K_REDUCE,      /* frame reduction of tile partials */
     FVGS_K_GN,          /* on-device Gauss-Newton pose update */
-    FVGS_K_MAP_FWD,     /* mapping forward with checkpoints */
-    FVGS_K_MAP_BWD,     /* mapping per-Gaussian backward */
+    FVGS_K_MAP_FWD,     /* mapping forward */
+    FVGS_K_MAP_BWD,     /* mapping backward */
     FVGS_K_MAP_UPDATE,  /* 2D->3D chain rule + Adam */
     FVGS_K_RENDER,      /* forward-only render */
     FVGS_K_MAINT,       /* map maintenance: visibility, outlier scores, marking, compaction */
@@ -370,7 +370,7 @@ int fvgs_render(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics* K
 
 /*
  * One mapping step against the frame of `level` seen from `pose`: binning,
- * forward blend with checkpoints, per-Gaussian backward to the 2D parameters,
+ * forward blend, backward to the 2D parameters of every Gaussian,
  * 2D->3D chain rule and an Adam update of every Gaussian parameter
  * (GSSlam::optimizeGaussiansKeyframe, src/GSSlam.cu:1083-1320, and its
  * kernels src/GSCudaKernels.cu:2074-2882; eta as eta_gaussian_).  Adam state

@@ -170,3 +170,33 @@ def test_render_view_list_and_block_edges(oracle, fvgs_lib, size, n, signed):
     both = crossed & crossed_o
     d = np.abs(dep[both] - dep_o[both]) / np.maximum(np.abs(dep_o[both]), 1.0)
     assert both.sum() == 0 or np.quantile(d, 0.99) <= 1e-5
+
+
+@pytest.mark.parametrize("signed", [False, True])
+@pytest.mark.parametrize("n", [33, 300])
+@pytest.mark.parametrize("size", [(477, 261), (640, 321)])
+def test_render_view_large_image_edges(oracle, fvgs_lib, size, n, signed):
+    """The form of images of more than three tiles per SM, cut by both edges; the
+    tolerances of the whole image."""
+    fv = fvgs_lib
+    W, H = size
+    K = (400.0, 400.0, (W - 1) / 2.0, (H - 1) / 2.0)
+    rng = np.random.default_rng(100 * n + W)
+    scene = S.cam_box(n, seed=n)
+    scene.positions[:, :2] = rng.uniform(-0.6, 0.6, (n, 2)) * scene.positions[:, 2:]
+    scene.scales[:] = rng.uniform(0.1, 0.4, (n, 3))
+    if signed:
+        scene.opacities[rng.random(n) < 0.1] *= -0.2
+    P = oracle.default_params(0x8)
+    pose = (np.zeros(3, np.float32), S.IDENTITY_Q)
+    b = oracle.prepare(scene, pose, K, W, H, P)
+    col_o, dep_o = oracle.render_view(scene, b, W, H, P)
+    with fv.Session(n, W, H, fv.default_params(0x8)) as s:
+        s.upload(scene)
+        col, dep, _ = s.render_view(pose, K, W, H, rgb8=True)
+    assert rel_err(col, col_o) <= 1e-5
+    crossed_o, crossed = dep_o < 1e9, dep < 1e9
+    assert (crossed != crossed_o).mean() <= 1e-4
+    both = crossed & crossed_o
+    d = np.abs(dep[both] - dep_o[both]) / np.maximum(np.abs(dep_o[both]), 1.0)
+    assert both.sum() == 0 or np.quantile(d, 0.999) <= 1e-5
