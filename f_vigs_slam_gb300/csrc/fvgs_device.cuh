@@ -191,6 +191,10 @@ __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// The same without letting the next kernel in early: for a grid that fills the
+// SMs' registers with CTAs that may have nothing to do.  The next kernel's CTAs,
+// waiting for room, would all settle on the few SMs whose CTAs leave first.
+__device__ __forceinline__ void pdl_begin_late() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // The conic's quadratic form v = a dx^2 + 2 b dx dy + c dy^2, evaluated as
 // dx * dl0 + dy * dl1 with dl0 = a dx + b dy, dl1 = b dx + c dy: the

@@ -771,7 +771,11 @@ template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) segsort_large_kernel(uint64_t* comp, uint64_t* tmp,
                                                                       const uint2* __restrict__ ranges, uint32_t* vals,
                                                                       SegSortWork w, DevStatus* st, SegSortIncr inc) {
-    pdl_begin();
+    // One CTA an SM with most of its registers, and usually no tile listed: let in
+    // early, the blending kernel crowded onto the SMs that were left first.  Late
+    // / early, us: frame of 50 k Gaussians VGA 2838 / 3124, of 1 M HD 3315 / 3395,
+    // view of 75 k at 160x120 129 / 161.
+    pdl_begin_late();
     constexpr int kCap = seg_cap<NT>();
     extern __shared__ uint64_t s_keys[];
     __shared__ uint32_t s_red[2 * NT / 32];
