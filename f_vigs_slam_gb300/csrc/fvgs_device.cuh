@@ -46,7 +46,7 @@ __device__ __forceinline__ void store_pair(float4* p, const float4& a, const flo
 // Device-side status word bits (session->status[0]); host reads after a step.
 constexpr uint32_t kErrOverflow = 1u << 0;  // instance capacity exceeded
 constexpr uint32_t kErrTimeout = 1u << 1;   // bounded wait gave up
-constexpr uint32_t kErrBounds = 1u << 2;    // index check failed (debug builds)
+constexpr uint32_t kErrBounds = 1u << 2;    // a tile's list does not hold its instances: the host repeats in full
 
 // Status block layout in device memory (u32 words).
 struct DevStatus {

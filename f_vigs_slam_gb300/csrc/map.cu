@@ -589,9 +589,9 @@ __global__ void __launch_bounds__(kUpdThreads) map_update_kernel(MapUpdateArgs a
     __shared__ int q_n;
     const int t = threadIdx.x, lane = t & 31;
     if (blockIdx.x == 0 && t < a.n_cst && a.cst) a.cst[t].valid = 0;
-    // An instance overflow leaves the binning incomplete; the host re-runs the
-    // step with larger buffers, so the parameters must stay untouched.
-    if (st->flags & kErrOverflow) return;
+    // After an instance overflow, or where a tile's list was not written, the
+    // host repeats the step or reports the error: the parameters stay untouched.
+    if (st->flags) return;
     if (t == 0) q_n = 0;
     __syncthreads();
     const int base = blockIdx.x * kUpdThreads * per;

@@ -58,3 +58,34 @@ def rel_err(a, b):
     b = np.asarray(b, np.float64)
     den = np.linalg.norm(b)
     return float(np.linalg.norm(a - b) / (den if den > 0 else 1.0))
+
+
+def crossing_layers(oracle_mod, n, K, W, H):
+    """n small Gaussians in one tile and two cameras at a right angle: in the
+    first one's depth order (which is the index order) the second one sees a near
+    and a far layer take turns.  The places that give both cameras these depths
+    are found by moving each Gaussian by the difference, a few times."""
+    from f_vigs_slam_gb300 import synthetic as S
+
+    scene = S.cam_box(n, seed=n)
+    scene.scales[:] = 0.005
+    scene.positions[:] = [0.0, 0.0, 2.0]
+    front = (np.zeros(3, np.float32), S.IDENTITY_Q)
+    side = (np.array([-2, 0, 2], np.float32), np.array([0, np.sqrt(0.5), 0, np.sqrt(0.5)], np.float32))
+    i = np.arange(n)
+    targets = ((front, 2, np.linspace(1.95, 2.05, n)), (side, 0, np.where(i % 2, 2.01, 1.94) + 0.05 * i / n))
+    P = oracle_mod.default_params()
+
+    def depths(pose):
+        b = oracle_mod.prepare(scene, pose, K, W, H, P)
+        assert b.keys.shape[0] == n
+        d = np.empty(n, np.float32)
+        d[b.vals] = (b.keys & np.uint64(0xffffffff)).astype(np.uint32).view(np.float32)
+        return d, b.vals
+
+    for _ in range(20):
+        for pose, axis, depth in targets:
+            scene.positions[:, axis] += depth - depths(pose)[0]
+    order = depths(front)[1]
+    assert depths(side)[0][order[:: n // 4096]].max() < 2.0  # n/4096 apart, all are of the near layer
+    return scene, front, side

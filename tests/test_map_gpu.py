@@ -5,10 +5,13 @@ Contract tolerance: Gaussian gradients within 1e-4 relative of the FP64
 oracle (Frobenius norm over all Gaussians, per DeltaGaussian2D / 3D field
 group).  The forward images share the tracking tolerance (1e-5).
 """
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
-from conftest import make_frame, rel_err, scaled_camera
+from conftest import ROOT, crossing_layers, make_frame, rel_err, scaled_camera
 from f_vigs_slam_gb300 import synthetic as S
 
 pytestmark = pytest.mark.gpu
@@ -138,3 +141,36 @@ def test_map_step_list_and_block_edges(oracle, fvgs_lib, size, n, quirks):
     for name, cols in GROUPS_2D.items():
         e = rel_err(g["delta2d"][same][:, cols], o.delta2d[same][:, cols])
         assert e <= GRAD_RTOL, (name, e)
+
+
+def test_update_leaves_the_map_after_a_failed_binning(fvgs_lib, tmp_path):
+    """The update writes nothing under any error flag of the step's binning: the
+    host repeats such a step, or reports it."""
+    from f_vigs_slam_gb300 import build
+
+    lib_dir = os.path.dirname(fvgs_lib.LIB_PATH)
+    exe = str(tmp_path / "map_update_flags")
+    cmd = [build.nvcc(), *build._flags(), os.path.join(ROOT, "tests", "cpp", "map_update_flags.cu"), "-L", lib_dir,
+           "-lfvgs", "-Xlinker", "-rpath," + lib_dir, "-o", exe]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    changed = dict(tuple(map(int, line.split())) for line in r.stdout.splitlines())
+    assert changed.pop(0) > 0
+    assert set(changed) == {1, 2, 4} and not any(changed.values()), changed
+
+
+def test_map_step_on_crossing_layers_steps_once(oracle, fvgs_lib):
+    """A carried-over list whose order is the worst for sampling: whatever the
+    binning makes of it, a mapping step that succeeds is one step of Adam."""
+    W, H, K = 16, 16, (40.0, 40.0, 7.5, 7.5)
+    scene, front, side = crossing_layers(oracle, 32768, K, W, H)
+    frame = make_frame(oracle, scene, side, K, W, H, oracle.default_params())
+    with fvgs_lib.Session(scene.n, W, H) as s:
+        s.upload(scene)
+        s.set_frame(0, *frame)
+        s.project_bin(front, K, W, H)
+        s.map_step(side, K, eta=1e-4)
+        steps = s.download_adam_state()[8, :, 2]
+    assert set(np.unique(steps)) == {0.0, 1.0}
