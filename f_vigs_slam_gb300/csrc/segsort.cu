@@ -14,9 +14,10 @@
 //    memory by distribution (sort_tile);
 //  * larger tiles (big maps, coarse pyramid levels) are listed by the first
 //    kernel and sorted by a second one with 1024 threads: up to 16384 instances
-//    the same way, beyond that split by key range -- 4096 sampled keys cut
-//    the tile into ranges, each of which a CTA collects from the whole source
-//    list (reading it twice, but all ranges at once and without exchange);
+//    the same way, beyond that split by key range -- 4096 sampled keys (or,
+//    where they miss most of the tile, exact ranks) cut the tile into ranges,
+//    each of which a CTA collects from the whole source list (reading it
+//    twice, but all ranges at once and without exchange);
 //  * tiles above 2^20 instances go to a merge sort through global memory.
 //
 // A list that has not changed (no member left or entered, keys still in
@@ -634,12 +635,81 @@ __device__ __forceinline__ bool source_key(const SegSortIncr& inc, const uint64_
     return rect_contains(b0, tx, ty);
 }
 
+// A tile's cut number `part`: a key with at most part * kPart keys of the tile
+// below it and fewer than kPart between it and that rank (`below`: the keys below
+// the cut).  The keys' bits are followed from the top, 12 a pass, into the bin
+// that holds the rank, until a bin holds at most kPart keys; its start is the cut.
+// The bins of two cuts are the same or apart, so cuts come in order, and keys
+// are unique, so the last bits leave one.  Whatever the keys and their order, two
+// neighbouring cuts enclose fewer than 2 kPart keys.  hist: kPartSamples + 4 words.
+// What bounds it: two to five more readings of the list for each of a range's
+// two cuts.  One tile of 65,536 entries, carried over: 279 us of sort, where the
+// samples serve 149; the binning repeated in full instead took 271 and could
+// fail again.
+template <int NT>
+__device__ __noinline__ uint64_t rank_cut(uint32_t* hist, uint32_t* s_red, uint32_t part, int n, const uint64_t* comp,
+                                          bool incr, const SegSortIncr& inc, uint32_t src0, int n_src, uint32_t enter0,
+                                          int n_all, int tx, int ty, uint32_t& below) {
+    constexpr int S = kPartSamples, PER = S / NT, kBits = 12;
+    static_assert(S == 1 << kBits, "a counter per value of the bits of a pass");
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const uint32_t kPart = part_keys<NT>(), rank = part * kPart;
+    uint32_t* bin = hist + S;  // [0] the bin, [1] keys below it, [2] keys in it
+    uint64_t prefix = 0;       // the bin so far: keys with these bits above `shift`
+    uint32_t count = (uint32_t)n;
+    int shift = 64;
+    below = 0;
+    while (count > kPart && shift > 0) {
+        const int bits = min(kBits, shift), down = shift - bits;
+        for (int k = t; k < S; k += NT) hist[k] = 0;
+        __syncthreads();
+        for (int i = t; i < n_all; i += NT) {
+            uint64_t key;
+            if (source_key(inc, comp, incr, src0, n_src, enter0, tx, ty, i, key) &&
+                (shift == 64 || key >> shift == prefix))
+                atomicAdd(&hist[(uint32_t)(key >> down) & ((1u << bits) - 1u)], 1u);
+        }
+        __syncthreads();
+        uint32_t sum = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) sum += hist[t * PER + k];
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_red[w] = incl;
+        __syncthreads();
+        uint32_t run = below + incl - sum;
+        for (int k = 0; k < w; ++k) run += s_red[k];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const uint32_t c = hist[t * PER + k];
+            if (rank >= run && rank - run < c) {
+                bin[0] = (uint32_t)(t * PER + k);
+                bin[1] = run;
+                bin[2] = c;
+            }
+            run += c;
+        }
+        __syncthreads();
+        prefix = prefix << bits | bin[0];
+        below = bin[1];
+        count = bin[2];
+        shift = down;
+        __syncthreads();  // the bin is read before the next pass writes it
+    }
+    return shift == 64 ? 0ull : prefix << shift;
+}
+
 // Range `part` of a large tile.  Every CTA of the tile samples and counts
 // alike: kPartSamples source keys in order are the splitters, the exact counts
 // between them give each segment's start, and range p holds the segments that
-// start in [p, p + 1) kPart.  Segments above kPart keys (sampling can
-// miss by that much only in tiles near kGlobalMin) are reported, and the host
-// repeats the binning in full.
+// start in [p, p + 1) kPart.  The samples stand at even places of the source
+// list, so where its order repeats with their distance (layers that alternate
+// from Gaussian to Gaussian) they miss most of the keys; a tile with a segment
+// above kPart keys is cut by rank instead.
 template <int NT>
 __device__ void sort_part(uint64_t* s_keys, uint32_t* s_red, uint32_t tile, uint32_t part, uint2 r, bool incr,
                           const uint64_t* __restrict__ comp, uint32_t* __restrict__ vals, DevStatus* st,
@@ -707,36 +777,51 @@ __device__ void sort_part(uint64_t* s_keys, uint32_t* s_red, uint32_t tile, uint
     const uint32_t wsum = lane < NT / 32 ? s_red[lane] : 0u;
     const uint32_t total = __reduce_add_sync(kFullMask, wsum);
     top = __reduce_max_sync(kFullMask, lane < NT / 32 ? s_red[NT / 32 + lane] : 0u);
-    if (total != (uint32_t)n || top > (uint32_t)kPart) {
+    if (total != (uint32_t)n) {
         if (t == 0) atomicOr(&st->flags, kErrBounds);
         return;
     }
-    // the range's first segment, its end and its first key's place
-    uint32_t run = __reduce_add_sync(kFullMask, lane < w ? wsum : 0u) + incl - sum;
     uint32_t* first = hist + S;  // [0] first segment, [1] end segment, [2] first place, [3] keys collected
-    __syncthreads();
-    if (t == 0) {
-        first[0] = S;
-        first[1] = 0;
-        first[2] = 0xffffffffu;
-        first[3] = 0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-        if (c[k] && run / kPart == part) {
-            atomicMin(&first[0], (uint32_t)(t * PER + k));
-            atomicMax(&first[1], (uint32_t)(t * PER + k + 1));
-            atomicMin(&first[2], run);
+    uint32_t below;              // the range's keys: lo <= key < hi (open: no end), the first one's place
+    uint64_t lo, hi = 0;
+    bool open;
+    if (top > (uint32_t)kPart) {
+        if (part * (uint32_t)kPart >= (uint32_t)n) return;
+        lo = rank_cut<NT>(hist, s_red, part, n, comp, incr, inc, src0, n_src, enter0, n_all, tx, ty, below);
+        open = (part + 1) * (uint32_t)kPart >= (uint32_t)n;
+        if (!open) {
+            uint32_t next;
+            hi = rank_cut<NT>(hist, s_red, part + 1, n, comp, incr, inc, src0, n_src, enter0, n_all, tx, ty, next);
         }
-        run += c[k];
+        if (t == 0) first[3] = 0;
+    } else {
+        // the range's first segment, its end and its first key's place
+        uint32_t run = __reduce_add_sync(kFullMask, lane < w ? wsum : 0u) + incl - sum;
+        __syncthreads();
+        if (t == 0) {
+            first[0] = S;
+            first[1] = 0;
+            first[2] = 0xffffffffu;
+            first[3] = 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            if (c[k] && run / kPart == part) {
+                atomicMin(&first[0], (uint32_t)(t * PER + k));
+                atomicMax(&first[1], (uint32_t)(t * PER + k + 1));
+                atomicMin(&first[2], run);
+            }
+            run += c[k];
+        }
+        __syncthreads();
+        const uint32_t s0 = first[0], s1 = first[1];
+        if (s1 == 0) return;  // no segment starts in this range
+        below = first[2];
+        lo = s0 ? s_keys[spad((int)s0 - 1)] : 0ull;
+        open = s1 >= (uint32_t)S;
+        if (!open) hi = s_keys[spad((int)s1 - 1)];
     }
-    __syncthreads();
-    const uint32_t s0 = first[0], s1 = first[1], below = first[2];
-    if (s1 == 0) return;  // no segment starts in this range
-    const uint64_t lo = s0 ? s_keys[spad((int)s0 - 1)] : 0ull;
-    const bool open = s1 >= (uint32_t)S;
-    const uint64_t hi = open ? 0ull : s_keys[spad((int)s1 - 1)];
     __syncthreads();  // the samples make room for the keys
     for (int i0 = 0; i0 < n_all; i0 += 4 * NT) {
         uint64_t key[4];
@@ -758,7 +843,10 @@ __device__ void sort_part(uint64_t* s_keys, uint32_t* s_red, uint32_t tile, uint
     }
     __syncthreads();
     const int cnt = (int)first[3];
-    if (cnt > seg_cap<NT>()) return;  // not reached: a range holds below 2 kPart keys
+    if (cnt > seg_cap<NT>()) {  // a range holds below 2 kPart keys unless the lists do not agree
+        if (t == 0) atomicOr(&st->flags, kErrBounds);
+        return;
+    }
     sort_tile<NT, kSegItems, kSrcShared>(SegShared<NT>(s_keys), s_red, tile, r.x + below, cnt, cnt, 0, comp, vals, st,
                                          inc);
 }
@@ -770,7 +858,8 @@ __device__ void sort_part(uint64_t* s_keys, uint32_t* s_red, uint32_t tile, uint
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) segsort_large_kernel(uint64_t* comp, uint64_t* tmp,
                                                                       const uint2* __restrict__ ranges, uint32_t* vals,
-                                                                      SegSortWork w, DevStatus* st, SegSortIncr inc) {
+                                                                      SegSortWork w, DevStatus* st,
+                                                                      const __grid_constant__ SegSortIncr inc) {
     // One CTA an SM with most of its registers, and usually no tile listed: let in
     // early, the blending kernel crowded onto the SMs that were left first.  Late
     // / early, us: frame of 50 k Gaussians VGA 2838 / 3124, of 1 M HD 3315 / 3395,

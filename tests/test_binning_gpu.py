@@ -7,7 +7,7 @@ sides use the same FP32 operation order).
 import numpy as np
 import pytest
 
-from conftest import scaled_camera
+from conftest import crossing_layers, scaled_camera
 from f_vigs_slam_gb300 import synthetic as S
 
 pytestmark = pytest.mark.gpu
@@ -151,3 +151,88 @@ def test_one_tile_sort_sizes(oracle, fvgs_lib, n, equal):
             np.testing.assert_array_equal(ranges, b.ranges)
             np.testing.assert_array_equal(vals, b.vals)
             np.testing.assert_array_equal(keys, b.keys)
+
+
+def _expect_binning(oracle, s, scene, pose, K, W, H):
+    n_inst = s.project_bin(pose, K, W, H)
+    b = oracle.prepare(scene, pose, K, W, H, oracle.default_params())
+    keys, vals, ranges = s.download_binning(W, H)
+    assert n_inst == b.keys.shape[0]
+    np.testing.assert_array_equal(ranges, b.ranges)
+    np.testing.assert_array_equal(vals, b.vals)
+    np.testing.assert_array_equal(keys, b.keys)
+    return b
+
+
+def _alternating(n, every, near, far):
+    """Two layers, the near one taking every `every`-th place, each spread over 0.05."""
+    i = np.arange(n)
+    return np.where(i % every == 0, near, far) + 0.05 * i / n
+
+
+@pytest.mark.parametrize("n,every", [(32768, 2), (40960, 2), (65536, 2), (65536, 16), (131072, 2), (131072, 32),
+                                     (262144, 64)])
+def test_one_tile_sort_alternating_layers(oracle, fvgs_lib, n, every):
+    """A tile above one CTA's capacity whose depths alternate with the Gaussian
+    index: samples at even places of its list may then all come from one layer,
+    and the other holds most of the tile between two of them."""
+    W, H, K = 16, 16, (40.0, 40.0, 7.5, 7.5)
+    rng = np.random.default_rng(n + every)
+    scene = S.cam_box(n, seed=n)
+    scene.scales[:] = 0.005
+    z = _alternating(n, every, 1.5, 2.5)
+    scene.positions[:] = np.stack([rng.uniform(-0.1, 0.1, n) * z, rng.uniform(-0.1, 0.1, n) * z, z], 1)
+    pose = (np.zeros(3, np.float32), S.IDENTITY_Q)
+    with fvgs_lib.Session(n, W, H) as s:
+        s.upload(scene)
+        for _ in range(2):
+            assert _expect_binning(oracle, s, scene, pose, K, W, H).keys.shape[0] == n
+        pose = S.perturb(pose, 0.5, 1.0, rng)
+        assert _expect_binning(oracle, s, scene, pose, K, W, H).keys.shape[0] == n
+
+
+@pytest.mark.parametrize("tiles", [1, 32])
+@pytest.mark.parametrize("n", [32768, 65536])
+def test_one_tile_sort_alternating_layers_incremental(oracle, fvgs_lib, n, tiles):
+    """The same for a list that is carried over and whose order the next camera
+    sees alternate.  With 32 tiles, all but one empty, the mean length picks the
+    sort's forms for short lists."""
+    W, H, K = (16, 16, (40.0, 40.0, 7.5, 7.5)) if tiles == 1 else (128, 64, (40.0, 40.0, 55.5, 23.5))
+    scene, front, side = crossing_layers(oracle, n, K, W, H)
+    with fvgs_lib.Session(n, W, H) as s:
+        s.upload(scene)
+        for k, pose in enumerate((front, side, front)):
+            _expect_binning(oracle, s, scene, pose, K, W, H)
+            assert bool(s.binning_info()["incremental"]) == (k > 0)
+
+
+@pytest.mark.parametrize("fill", [100, 1200])
+@pytest.mark.parametrize("dense", [2049, 4097, 8193, 16384, 20000])
+def test_dense_tile_among_short_lists(oracle, fvgs_lib, dense, fill):
+    """One tile far above the grid's mean, which picks the sort's forms for
+    short lists (means up to 1024 and 2048) once a binning has set it; the dense
+    tile's layers alternate by index.  A re-upload makes a full binning."""
+    W, H, K = 128, 64, (40.0, 40.0, 63.5, 31.5)
+    tiles = [(tx, ty) for ty in range(4) for tx in range(8)]
+    n_tile = [dense if t == (3, 1) else fill for t in tiles]
+    order = sorted(range(len(tiles)), key=lambda k: tiles[k] != (3, 1))  # the dense tile's Gaussians first
+    n = sum(n_tile)
+    rng = np.random.default_rng(dense + fill)
+    scene = S.cam_box(n, seed=dense)
+    scene.scales[:] = 0.005
+    at = np.concatenate([np.tile(tiles[k], (n_tile[k], 1)) for k in order])
+    uv = 16.0 * at + 8.0 + rng.uniform(-0.5, 0.5, (n, 2))
+    z = np.concatenate([_alternating(dense, 2, 1.8, 2.2), rng.uniform(1.5, 2.5, n - dense)])
+    scene.positions[:] = np.stack([(uv[:, 0] - K[2]) / K[0] * z, (uv[:, 1] - K[3]) / K[1] * z, z], 1)
+    poses = [(np.zeros(3, np.float32), S.IDENTITY_Q)]
+    for deg, cm in ((0.0, 0.0), (0.05, 0.1), (0.3, 1.0)):
+        poses.append(S.perturb(poses[-1], deg, cm, rng))
+    with fvgs_lib.Session(n, W, H) as s:
+        s.upload(scene)
+        b = _expect_binning(oracle, s, scene, poses[0], K, W, H)
+        assert b.keys.shape[0] // len(tiles) <= (1024 if fill < 1000 else 2048)
+        assert (b.ranges[:, 1] - b.ranges[:, 0]).max() >= dense
+        s.upload(scene)
+        for pose in poses:
+            _expect_binning(oracle, s, scene, pose, K, W, H)
+            _expect_binning(oracle, s, scene, pose, K, W, H)
