@@ -1576,17 +1576,15 @@ namespace {
 // CUDA events on the session's stream), keep the fastest median for frames
 // of this shape.  Every variant computes the same values in the same order,
 // so the choice changes only the time.
-// Whether launch variant v is a distinct choice for the level's frames: the
-// split ones need 16 x 16 tiles without compensated sums.
+// Whether launch variant v is a distinct choice for the level's frames:
+// compensated sums and the other tile shapes have one form, variant 0.
 bool variant_applies(const fvgs_session* s, const FrameLevel& f, int v) {
-    if (track_variant_split(v) > 1) {
-        TrackArgs a{};
-        a.tile_w = f.tile_w ? f.tile_w : 16;
-        a.tile_h = f.tile_h ? f.tile_h : 16;
-        a.compensated = s->precision == FVGS_PRECISION_REDUCED && !(s->params.quirks & FVGS_Q_POSE_JAC_APPROX);
-        return split_ok(a);
-    }
-    return true;
+    if (v == 0) return true;
+    TrackArgs a{};
+    a.tile_w = f.tile_w ? f.tile_w : 16;
+    a.tile_h = f.tile_h ? f.tile_h : 16;
+    a.compensated = s->precision == FVGS_PRECISION_REDUCED && !(s->params.quirks & FVGS_Q_POSE_JAC_APPROX);
+    return split_ok(a);
 }
 
 int autotune_track(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics* K, int level, int reps) {
@@ -1626,11 +1624,12 @@ int autotune_track(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics
     }
     float med[kTrackVariants] = {};
     if (rc == FVGS_OK) {
-        for (int v = 0; v < kTrackVariants; ++v) {
+        for (int v = 0; v < kTrackVariants && rc == FVGS_OK; ++v) {
+            if (!variant_applies(s, f, v)) continue;  // its events were not recorded
             std::vector<float> t(reps);
             for (int r = 0; r < reps; ++r) {
                 const size_t k = 2 * ((size_t)r * kTrackVariants + v);
-                cudaEventElapsedTime(&t[r], ev[k], ev[k + 1]);
+                if (cudaEventElapsedTime(&t[r], ev[k], ev[k + 1]) != cudaSuccess) rc = FVGS_E_CUDA;
             }
             std::sort(t.begin(), t.end());
             med[v] = t[reps / 2];

@@ -121,7 +121,8 @@ int fvgs_session_set_precision(fvgs_session* s, int precision);
  * depend on the choice.
  * fvgs_session_autotune runs the tuning explicitly (reps timed launches per
  * variant; variant and per-variant median ms (FVGS_TRACK_VARIANTS floats) may
- * be null); fvgs_session_set_autotune(s, 0) keeps variant 0 for untuned
+ * be null; where there is one form, that is variant 0, and the others report
+ * 0 ms); fvgs_session_set_autotune(s, 0) keeps variant 0 for untuned
  * shapes; fvgs_session_set_track_variant restores a known choice.  No
  * reference counterpart.
  */

@@ -95,3 +95,30 @@ def test_split_tiles_give_the_same_tile_partials(oracle, fvgs_lib, analytic):
     for v in (5, 6):
         for x, y in zip(out[0], out[v]):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("form", ["compensated", "8x8", "32x8"])
+def test_shapes_of_one_form(oracle, fvgs_lib, form):
+    """Compensated sums and tiles of 8 x 8 and 32 x 8 have one launch form: the
+    tuner times it as variant 0, reports 0 ms for the others, and leaves no
+    error behind for the calls after it."""
+    fv = fvgs_lib
+    W, H, K = scaled_camera(0.25)
+    scene = S.cam_box(5_000, seed=77)
+    quirks = fv.QUIRKS_INTENDED
+    pose = (np.zeros(3), S.IDENTITY_Q)
+    frame = make_frame(oracle, scene, pose, K, W, H, oracle.default_params(quirks))
+    with fv.Session(scene.n, W, H, fv.default_params(quirks)) as s:
+        s.upload(scene)
+        s.set_frame(0, *frame)
+        if form == "compensated":
+            s.set_precision(fv.PRECISION_REDUCED)
+        else:
+            s.set_track_tiles(0, *map(int, form.split("x")))
+        s.set_timing(["track"])
+        v, ms = s.autotune(pose, K, 0, reps=3)
+        launches = s.get_timing(reset=True)["track"]["launches"]
+        s.upload(scene)
+        s.track_frame(pose, K, iterations=1)
+        assert v == 0 and ms[0] > 0 and not ms[1:].any(), (v, ms)
+        assert launches == 3
