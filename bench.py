@@ -1267,9 +1267,8 @@ def run_batching(args, fvgs, S, torch, dev, world):
         w["sess"].close()
     seq_s, bat_s, str_s = max_over_ranks([seq_s, bat_s, str_s], dev, world)
     n = steps * len(ws)
-    levels = {"level%d" % l: {"tile": "%dx%d" % c[:2], "smem_batch": c[2],
-                              "ms_per_launch": {"%dx%d" % sh: {str(bb): round(float(tuned_ms[l][i][j]), 4)
-                                                              for j, bb in enumerate(fvgs.STAGE_BATCHES)}
+    levels = {"level%d" % l: {"tile": "%dx%d" % c[:2],
+                              "ms_per_launch": {"%dx%d" % sh: round(float(tuned_ms[l][i][0]), 4)
                                                 for i, sh in enumerate(fvgs.TILE_SHAPES)}}
               for l, c in sorted(tuned.items())}
     return {"workload": "%d keyframes, N log-uniform in [20k, 2M] (%d Gaussians in total), 640x480 / 1280x720, "

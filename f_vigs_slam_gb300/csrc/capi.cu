@@ -2100,7 +2100,7 @@ struct fvgs_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_fork = nullptr;
     std::vector<cudaEvent_t> ev_join;
-    int tw[kMaxLevels], th[kMaxLevels], variant[kMaxLevels];
+    int tw[kMaxLevels], th[kMaxLevels];
     uint32_t* counters = nullptr;  // the persistent kernel's work counters
     // job tables, one region per Gauss-Newton iteration: host (pinned)
     // staging, the eager path's device copy and the captured frame's
@@ -2123,7 +2123,7 @@ struct fvgs_batch {
     struct Graph {
         bool valid = false;
         int iters[kMaxLevels] = {};
-        int tw[kMaxLevels] = {}, th[kMaxLevels] = {}, variant[kMaxLevels] = {};
+        int tw[kMaxLevels] = {}, th[kMaxLevels] = {};
         std::vector<Exit> exit;
         uint64_t batch_launches = 0;
         cudaGraphExec_t exec = nullptr;
@@ -2177,19 +2177,27 @@ int batch_ensure_tables(fvgs_batch* b, int iters) {
     return FVGS_OK;
 }
 
+// The staging batch (Gaussians) that a tuned level reports; it reaches no kernel.
+constexpr int kStageBatch = 256;
+
 // Push a level's tile shape to every session, so each one's plain frames
-// blend exactly as the batch does.
+// blend exactly as the batch does; captured frames stay where nothing changes.
 void batch_apply_level(fvgs_batch* b, int l) {
+    bool changed = false;
     for (fvgs_session* s : b->s) {
         FrameLevel& f = s->lv[l];
+        if (f.tile_w == b->tw[l] && f.tile_h == b->th[l] && f.track_variant == 0 && f.tuned_w == f.W &&
+            f.tuned_h == f.H)
+            continue;
         f.tile_w = b->tw[l];
         f.tile_h = b->th[l];
         f.track_variant = 0;
         f.tuned_w = f.W;
         f.tuned_h = f.H;
         ++s->gen;
+        changed = true;
     }
-    batch_drop_graph(b);
+    if (changed) batch_drop_graph(b);
 }
 
 // Fork the sessions' streams off the batch stream / join them back.
@@ -2289,9 +2297,7 @@ bool batch_key_matches(fvgs_batch* b, const Request* reqs) {
     const fvgs_batch::Graph& g = b->graph;
     if (!g.valid) return false;
     for (int l = 0; l < kMaxLevels; ++l)
-        if (g.iters[l] != reqs[0].iters[l] || g.tw[l] != b->tw[l] || g.th[l] != b->th[l] ||
-            g.variant[l] != b->variant[l])
-            return false;
+        if (g.iters[l] != reqs[0].iters[l] || g.tw[l] != b->tw[l] || g.th[l] != b->th[l]) return false;
     for (size_t i = 0; i < b->s.size(); ++i) {
         fvgs_session* s = b->s[i];
         const fvgs_batch::Exit& e = g.exit[i];
@@ -2434,7 +2440,6 @@ int batch_launch(fvgs_batch* b, const Request* reqs) {
         g.iters[l] = reqs[0].iters[l];
         g.tw[l] = b->tw[l];
         g.th[l] = b->th[l];
-        g.variant[l] = b->variant[l];
     }
     g.exit = exit;
     g.batch_launches = b->batch_launches - launches0;
@@ -2477,10 +2482,7 @@ int fvgs_batch_create(fvgs_session* const* sessions, int n, fvgs_batch** out) {
     b->device = sessions[0]->device;
     b->num_sms = sessions[0]->num_sms;
     b->analytic = !(sessions[0]->params.quirks & FVGS_Q_POSE_JAC_APPROX);
-    for (int l = 0; l < kMaxLevels; ++l) {
-        b->tw[l] = b->th[l] = 16;
-        b->variant[l] = 0;
-    }
+    for (int l = 0; l < kMaxLevels; ++l) b->tw[l] = b->th[l] = 16;
     b->ev_join.assign(n, nullptr);
     bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
@@ -2517,7 +2519,6 @@ int fvgs_batch_set_level(fvgs_batch* b, int level, int tile_w, int tile_h, int b
     if (batch_gaussians != 128 && batch_gaussians != 256 && batch_gaussians != 512) return FVGS_E_INVALID;
     b->tw[level] = tile_w;
     b->th[level] = tile_h;
-    b->variant[level] = batch_gaussians == 128 ? 3 : (batch_gaussians == 512 ? 4 : 0);
     batch_apply_level(b, level);
     return FVGS_OK;
 }
@@ -2564,7 +2565,6 @@ int fvgs_batch_autotune(fvgs_batch* b, const fvgs_pose* poses, const fvgs_intrin
     reps = std::max(1, std::min(reps, 16));
     const size_t n = b->s.size();
     const int shapes[3][2] = {{16, 16}, {8, 8}, {32, 8}};
-    const int variants[3] = {3, 0, 4};  // batches of 128, 256, 512
     std::vector<cudaEvent_t> ev(2 * (size_t)reps, nullptr);
     for (auto& e : ev)
         if (cudaEventCreate(&e) != cudaSuccess) {
@@ -2577,7 +2577,7 @@ int fvgs_batch_autotune(fvgs_batch* b, const fvgs_pose* poses, const fvgs_intrin
     for (int l = 0; l < levels && l < kMaxLevels && rc == FVGS_OK; ++l) {
         if (reqs[0].iters[l] == 0) continue;
         float best = INFINITY;
-        int best_shape = 0, best_variant = 0;
+        int best_shape = 0;
         for (int sh = 0; sh < 3 && rc == FVGS_OK; ++sh) {
             b->tw[l] = shapes[sh][0];
             b->th[l] = shapes[sh][1];
@@ -2617,42 +2617,37 @@ int fvgs_batch_autotune(fvgs_batch* b, const fvgs_pose* poses, const fvgs_intrin
                 rc = FVGS_E_CUDA;
                 break;
             }
-            for (int vi = 0; vi < 3 && rc == FVGS_OK; ++vi) {
-                const int v = variants[vi];
-                for (int r = 0; r < reps && rc == FVGS_OK; ++r) {
-                    if (cudaEventRecord(ev[2 * r], b->stream) != cudaSuccess ||
-                        launch_track_batch(b->d_jobs, b->d_begin, (int)n, total, b->tw[l], b->th[l], b->analytic,
-                                           b->counters, b->num_sms, b->stream) != cudaSuccess ||
-                        cudaEventRecord(ev[2 * r + 1], b->stream) != cudaSuccess)
-                        rc = FVGS_E_CUDA;
-                }
-                if (rc == FVGS_OK && cudaStreamSynchronize(b->stream) != cudaSuccess) rc = FVGS_E_CUDA;
-                if (rc != FVGS_OK) break;
-                std::vector<float> t(reps);
-                for (int r = 0; r < reps; ++r) cudaEventElapsedTime(&t[r], ev[2 * r], ev[2 * r + 1]);
-                std::sort(t.begin(), t.end());
-                const float med = t[reps / 2];
-                if (ms_out) ms_out[l * 9 + sh * 3 + vi] = med;
-                // A shape other than the reference's 16 x 16 has to be a quarter
-                // faster: it blends other lists (its own rectangles and
-                // tile-centre depths), and the launch timed here leaves out
-                // its binning (8 x 8 tiles list 2.5 times the instances).
-                const float cost = sh == 0 ? med : 1.25f * med;
-                if (cost < best) {
-                    best = cost;
-                    best_shape = sh;
-                    best_variant = v;
-                }
+            for (int r = 0; r < reps && rc == FVGS_OK; ++r) {
+                if (cudaEventRecord(ev[2 * r], b->stream) != cudaSuccess ||
+                    launch_track_batch(b->d_jobs, b->d_begin, (int)n, total, b->tw[l], b->th[l], b->analytic,
+                                       b->counters, b->num_sms, b->stream) != cudaSuccess ||
+                    cudaEventRecord(ev[2 * r + 1], b->stream) != cudaSuccess)
+                    rc = FVGS_E_CUDA;
+            }
+            if (rc == FVGS_OK && cudaStreamSynchronize(b->stream) != cudaSuccess) rc = FVGS_E_CUDA;
+            if (rc != FVGS_OK) break;
+            std::vector<float> t(reps);
+            for (int r = 0; r < reps; ++r) cudaEventElapsedTime(&t[r], ev[2 * r], ev[2 * r + 1]);
+            std::sort(t.begin(), t.end());
+            const float med = t[reps / 2];
+            if (ms_out) std::fill_n(ms_out + l * 9 + sh * 3, 3, med);  // one time for every staging batch
+            // A shape other than the reference's 16 x 16 has to be a quarter
+            // faster: it blends other lists (its own rectangles and
+            // tile-centre depths), and the launch timed here leaves out
+            // its binning (8 x 8 tiles list 2.5 times the instances).
+            const float cost = sh == 0 ? med : 1.25f * med;
+            if (cost < best) {
+                best = cost;
+                best_shape = sh;
             }
         }
         if (rc != FVGS_OK) break;
         b->tw[l] = shapes[best_shape][0];
         b->th[l] = shapes[best_shape][1];
-        b->variant[l] = best_variant;
         if (config_out) {
             config_out[3 * l] = b->tw[l];
             config_out[3 * l + 1] = b->th[l];
-            config_out[3 * l + 2] = track_variant_batch(best_variant);
+            config_out[3 * l + 2] = kStageBatch;
         }
     }
     for (auto& e : ev) cudaEventDestroy(e);

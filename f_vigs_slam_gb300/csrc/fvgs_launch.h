@@ -263,9 +263,6 @@ constexpr int kTrackVariants = 8;
 inline bool track_tile_supported(int tw, int th) {
     return (tw == 16 && th == 16) || (tw == 8 && th == 8) || (tw == 32 && th == 8);
 }
-// The staging batch that a batch's level reports (fvgs_batch_set_level): 3 ->
-// 128, 4 -> 512, otherwise 256.
-inline int track_variant_batch(int variant) { return variant == 3 ? 128 : (variant == 4 ? 512 : 256); }
 // CTAs per 16 x 16 list tile of a launch variant: 4 (8 x 8 pixel quarters), 2
 // (16 x 8 halves) or 1.
 inline int track_variant_split(int variant) {

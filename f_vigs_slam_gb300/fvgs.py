@@ -613,7 +613,7 @@ class Batch:
                                              C.c_int(batch)), "fvgs_batch_set_level")
 
     def autotune(self, poses, K0s, iterations=(4, 4, 6, 6), reps: int = 5):
-        """Per level: the fastest (tile_w, tile_h, batch) and the 9 medians (ms, shape-major)."""
+        """Per level: the fastest (tile_w, tile_h, 256) and the shapes' medians (ms; 3 x 3, a row per shape)."""
         n = len(self.sessions)
         ps = (Pose * n)(*[make_pose(p) for p in poses])
         ks = (Intrinsics * n)(*[make_intr(k) for k in K0s])

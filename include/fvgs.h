@@ -305,17 +305,16 @@ int fvgs_session_set_track_tiles(fvgs_session* s, int level, int tile_w, int til
  * Each level's tile shape belongs to the batch and is pushed to its sessions
  * (fvgs_session_set_track_tiles), so a session's plain frames give the
  * batched result bit for bit.  The staging batch (128, 256 or 512 Gaussians)
- * is accepted and reported, and changes neither results nor the launch: every
- * warp stages 32 list entries at a time.  fvgs_batch_set_level sets both;
- * fvgs_batch_autotune times the persistent launch for every shape x
- * batch (9 combinations) on every level the schedule uses, at the given
- * poses (reps launches each), and keeps the fastest per level (another shape
- * than 16 x 16 only when it is a quarter faster); config_out
- * (nullable, 3 ints per level: tile_w, tile_h, batch) and ms_out (nullable,
- * 9 floats per level: shapes 16x16, 8x8, 32x8, each with batches 128, 256,
- * 512) report the outcome.  fvgs_batch_stats: frames replayed / enqueued
- * eagerly, batched kernel launches.  The reference tracks one frame of one
- * map per launch; no counterpart.
+ * is accepted and has no effect: every warp stages 32 list entries at a time.
+ * fvgs_batch_set_level sets a level's shape; fvgs_batch_autotune times the
+ * persistent launch for every shape on every level the schedule uses, at the
+ * given poses (reps launches each), and keeps the fastest per level (another
+ * shape than 16 x 16 only when it is a quarter faster); config_out
+ * (nullable, 3 ints per level: tile_w, tile_h, batch, the last always 256) and
+ * ms_out (nullable, 9 floats per level: shapes 16x16, 8x8, 32x8, each one's
+ * time in three places, one per batch) report the outcome.  fvgs_batch_stats:
+ * frames replayed / enqueued eagerly, batched kernel launches.  The reference
+ * tracks one frame of one map per launch; no counterpart.
  */
 typedef struct fvgs_batch fvgs_batch;
 int fvgs_batch_create(fvgs_session* const* sessions, int n, fvgs_batch** out);

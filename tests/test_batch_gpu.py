@@ -170,3 +170,20 @@ def test_batch_instance_overflow_and_reduced_precision(fvgs_lib):
         for p, q in zip(run, plain):
             np.testing.assert_array_equal(p[0], q[0])
             np.testing.assert_array_equal(p[1], q[1])
+
+
+def test_batch_staging_size_is_not_tuned(fvgs_lib):
+    """The staging batch reaches no kernel: a shape is timed once, its time stands
+    for all three sizes, and the size reported is the default."""
+    fv = fvgs_lib
+    ws = _sessions(fv, INTENDED, [(20_000, S.CAM_VGA), (40_000, S.CAM_VGA)], 90)
+    try:
+        with fv.Batch([w["s"] for w in ws]) as bt:
+            bt.set_level(0, 16, 16, 512)
+            cfg, ms = bt.autotune([w["start"] for w in ws], [w["K0"] for w in ws], PYR, reps=3)
+    finally:
+        for w in ws:
+            w["s"].close()
+    for l, m in ms.items():
+        np.testing.assert_array_equal(m, np.tile(m[:, :1], 3))
+        assert cfg[l][2] == 256
