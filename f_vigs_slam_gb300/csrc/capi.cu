@@ -17,7 +17,6 @@
 #include <new>
 #include <vector>
 
-
 #include "../../include/fvgs.h"
 #include "fvgs_device.cuh"
 #include "fvgs_launch.h"
@@ -242,8 +241,6 @@ struct fvgs_session {
     // precision form: reduced-precision copies of scale/rotation and
     // colour/opacity that the projection reads; the float4 planes stay the
     // master copy (mapping updates both)
-    // tensor maps of the record planes (TMA-staged Jacobian variant)
-
     int precision = FVGS_PRECISION_FP32;
     bool autotune = true;  // tune the Jacobian kernel's launch variant on a frame shape's first frame
     uint4* attr_sr = nullptr;
@@ -2781,7 +2778,6 @@ int fvgs_map_step(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics*
     const FrameLevel& f = s->lv[level];
     if (!f.rgb) return FVGS_E_STATE;
     FV_CK(cudaSetDevice(s->device));
-    const bool cap = (s->params.quirks & FVGS_Q_MAP_CAP256) != 0;
     FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H));
     for (int attempt = 0; attempt < 4; ++attempt) {
         FV_TRY(reset_status(s));
@@ -2793,11 +2789,7 @@ int fvgs_map_step(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics*
         collect_timing(s);
         int retry = 0;
         FV_TRY(check_status(s, &retry));
-        if (retry) {
-            // the instance buffers grew
-            FV_TRY(ensure_map_buffers(s, (size_t)f.W * f.H));
-            continue;
-        }
+        if (retry) continue;
         s->has_map = true;
         return FVGS_OK;
     }
