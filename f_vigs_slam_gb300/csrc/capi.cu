@@ -1568,11 +1568,6 @@ int fvgs_download_track_images(fvgs_session* s, float* color, float* depth, floa
 
 namespace {
 
-// Launch-variant autotuner of the Jacobian kernel: bin the level's frame at
-// `pose`, run every variant `reps` times in turn on that binning (timed with
-// CUDA events on the session's stream), keep the fastest median for frames
-// of this shape.  Every variant computes the same values in the same order,
-// so the choice changes only the time.
 // Whether launch variant v is a distinct choice for the level's frames:
 // compensated sums and the other tile shapes have one form, variant 0.
 bool variant_applies(const fvgs_session* s, const FrameLevel& f, int v) {
@@ -1584,6 +1579,11 @@ bool variant_applies(const fvgs_session* s, const FrameLevel& f, int v) {
     return split_ok(a);
 }
 
+// Launch-variant autotuner of the Jacobian kernel: bin the level's frame at
+// `pose`, run every distinct variant `reps` times in turn on that binning (timed with
+// CUDA events on the session's stream), keep the fastest median for frames
+// of this shape.  Every variant computes the same values in the same order,
+// so the choice changes only the time.
 int autotune_track(fvgs_session* s, const fvgs_pose* pose, const fvgs_intrinsics* K, int level, int reps) {
     FrameLevel& f = s->lv[level];
     if (!f.rgb) return FVGS_E_STATE;
